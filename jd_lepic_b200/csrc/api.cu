@@ -49,7 +49,7 @@ static void free_all(lepic_ctx *c) {
     }
     F(c->keys); F(c->perm); F(c->counts); F(c->offsets); F(c->cursor); F(c->blocksums); F(c->bigseg);
     for (int l = 0; l < c->nlev; l++) {
-        if (l > 0) { F(c->lev[l].u); F(c->lev[l].b); F(c->lev[l].bc); }
+        if (l > 0) { F(c->lev[l].u); F(c->lev[l].u2); F(c->lev[l].b); F(c->lev[l].bc); }
         F(c->lev[l].e32); F(c->lev[l].e32b); F(c->lev[l].r32);
         F(c->lev[l].e64); F(c->lev[l].e64b); F(c->lev[l].r64);
     }
@@ -205,7 +205,7 @@ static int create_impl(lepic_ctx *c, const lepic_config *cfg, const int32_t *bcn
             cur[L.nx + 2] = prev[nxf + 2];
             cur[(L.ny + 2) * W2] = prev[(nyf + 2) * Wf];
             cur[L.nx + 2 + (L.ny + 2) * W2] = prev[nxf + 2 + (nyf + 2) * Wf];
-            LALLOC(L.u, nnl); LALLOC(L.b, (size_t)(L.nx + 1) * (L.ny + 1)); LALLOC(L.bc, nnl + 16);
+            LALLOC(L.u, nnl); LALLOC(L.u2, nnl + L.ny + 3); LALLOC(L.b, (size_t)(L.nx + 1) * (L.ny + 1)); LALLOC(L.bc, nnl + 16);
             LCUDA(cudaMemset(L.u, 0, sizeof(double) * nnl));
             LCUDA(cudaMemset(L.b, 0, sizeof(double) * (L.nx + 1) * (L.ny + 1)));
             LCUDA(cudaMemcpy(L.bc, cur.data(), nnl, cudaMemcpyHostToDevice));
@@ -219,7 +219,8 @@ static int create_impl(lepic_ctx *c, const lepic_config *cfg, const int32_t *bcn
     // grid-wide sums: up to 3 values x 2 halves per CTA of a cooperative grid of at most 8 CTAs
     // of 256 threads per SM
     LALLOC(c->partials, (size_t)c->num_sms * 48);
-    LALLOC(c->cg_r, nn); LALLOC(c->cg_p, nn); LALLOC(c->cg_ap, nn);
+    // cg_ap: also the FP64 multigrid's second level-0 buffer, whose rows may be one node longer
+    LALLOC(c->cg_r, nn); LALLOC(c->cg_p, nn); LALLOC(c->cg_ap, nn + ny + 3);
     LCUDA(cudaMemset(c->cg_r, 0, sizeof(double) * nn));
     LCUDA(cudaMemset(c->cg_p, 0, sizeof(double) * nn));
     LCUDA(cudaMemset(c->cg_ap, 0, sizeof(double) * nn));

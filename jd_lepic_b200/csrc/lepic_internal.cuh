@@ -108,6 +108,7 @@ struct MGLevel {
     int nx, ny;
     double hx, hy;
     double *u;       // (nx+3)(ny+3)
+    double *u2;      // the FP64 multigrid's second buffer (level 0 uses the CG vector cg_ap)
     double *b;       // (nx+1)(ny+1)
     int8_t *bc;      // (nx+3)(ny+3), bcnd clamped to [-4, 1]
     float *e32;      // mixed precision correction (nx+3)(ny+3)
@@ -322,9 +323,9 @@ __device__ __forceinline__ int ld_volatile_i32(const int *p) {
     asm volatile("ld.volatile.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long *p) {
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long *p) {
     unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 // Each CTA adds one arrival to a counter that only grows during the launch (zeroed before it):
@@ -343,7 +344,7 @@ __device__ __forceinline__ bool grid_barrier(DevCounters *c, unsigned int nblock
         const unsigned long long nb = nblocks;
         const unsigned long long target = (atomicAdd(&c->bar_arrived, 1ull) / nb + 1) * nb;
         long long t0 = clock64();
-        while (ld_acquire_u64(&c->bar_arrived) < target) {
+        while (ld_relaxed_u64(&c->bar_arrived) < target) {
             if (ld_volatile_i32(&c->abort_flag) != 0) { ok = 0; break; }
             if (clock64() - t0 > 4000000000LL) {
                 set_err(c, LERR_TIMEOUT, 900);
@@ -411,7 +412,6 @@ int field_calc_efield(lepic_ctx *c);
 int field_np_grid(lepic_ctx *c, int ptype, double *d_out);
 int mg_solve(lepic_ctx *c, double eps, int mode);
 int mg_init(lepic_ctx *c);
-int mg_residual_stats(lepic_ctx *c);
 // the Bohm speed map of the 3rd-dimension model from an averaging sample (walls.cu)
 int zloss_after_avg(lepic_ctx *c, const double *data, int na1, int na2, int size_na, int cnt);
 // refluxing at x = 0 (sources.cu): true when the sources' opt_inj is +-4 and the Neumann option

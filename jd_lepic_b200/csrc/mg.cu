@@ -5,14 +5,25 @@
 // Compiled with -fmad=false: the SOR update, the residual and the restriction weights are
 // rounded exactly as the Fortran expressions are written, so with the same sweep counts the
 // result equals the FP64 CPU restatement bit for bit.  The L1 residual sums are reduced in a
-// fixed order (per-thread, fixed block tree, fixed cross-block order), so a solve is
-// reproducible run to run.
+// fixed order (per-thread, warp tree, warps, CTAs), so a solve is reproducible run to run.
 //
-// Levels whose node count is at most `small_nodes` are processed by CTA 0 alone with
-// block barriers; larger levels use the whole cooperative grid with a bounded software grid
-// barrier.  Roofline: each fine-level half-sweep streams u (8 B, 5-point), b (8 B) and the
-// int8 mask; at 2049^2 nodes the working set (u, b, mask: ~72 MB) is L2-resident, so the fine
-// sweeps are L2-bandwidth bound and the coarse levels are barrier-latency bound.
+// What bounds it: not bytes (a 513^2 level and its right-hand side are 4 MB, in L2) but the
+// chain of dependent steps.  The reference decides after every sweep whether to go on, so a
+// sweep run grid-wide costs three grid barriers (red, black, residual) of about 2-3 us, and a
+// sweep of a coarse level by one CTA out of global memory about 10 us.  So:
+//  * Levels above the CTA-0 part are swept in shared-memory tiles (temporal blocking): a CTA
+//    loads a tile of u, b and the mask with a halo, runs all K sweeps of a stage there (half-
+//    sweep h updates the nodes at least h + 1 nodes inside the region, so the tile ends with
+//    exactly the values of grid-wide sweeps), sums each sweep's residual on the way, and
+//    restricts the result into the next level's right-hand side in the same pass (or starts
+//    from the prolongation of the coarser correction): one grid barrier per stage.  K is the
+//    number of sweeps the stage took in the previous cycle.  The decisions are taken afterwards
+//    from the K sums, which are the reference's: if it would have stopped earlier, the pass is
+//    run again from its untouched input with that many sweeps; if not yet, another pass follows.
+//  * Levels of at most small_nodes nodes live in CTA 0's shared memory (u, b, mask) for the
+//    whole solve.
+// Measured (B200, warm solve to 1e-8, 4 cycles): 129^2 nodes 2.32 -> 1.02 ms, 513^2 3.05 -> 1.78 ms,
+// 384 x 256 cells with periodic edges 3.43 -> 1.56 ms; 513^2 cold to the L1 1e-10 4.96 -> 2.51 ms.
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -21,10 +32,12 @@
 struct MGDev {
     int nx, ny;
     double aw, an, ac;    // mg.h:11-15 (ae = aw, as = an)
-    double hx, hy;
-    double *u;
+    double y;             // 1 / ac (0: ac out of the range of quot())
+    double *u, *u2;       // the level's two buffers: a pass reads one and writes the other
     double *b;
     const int8_t *bc;
+    int tx, ty;           // the tile of the level's passes
+    int su, sb, sm;       // levels of the CTA-0 part: offsets of u, b and the mask in shared memory
 };
 
 struct MGP {
@@ -32,325 +45,820 @@ struct MGP {
     int ng, Ls;           // levels >= Ls are handled by CTA 0
     double omega, eps, alpha;
     int ncycl, pbc, nmn, mode;
+    int cap;              // nodes a tile's region may hold
     double *partials;
     DevCounters *cnt;
     unsigned bar_extra;        // lepic_options::barrier_extra
 };
 
-#include "mg_common.cuh"
+#define MGT 512           // threads per CTA, two CTAs per SM
+#define MGW (MGT / 32)
+#define MG_KMAX 4         // sweeps per pass
+#define MG_HMAX (2 * MG_KMAX + 2)
+#define MG_NSUM (MG_KMAX + 2)   // a pass's sums: |r| per sweep, r^2 after the last, ||b0||^2
+#define MG_NR 10          // sweeps per stage at most (but the coarsest level's in the first cycle)
 
-// ---------------------------------------------------------------------------------------
-// sors.f90:80-118 / :210-248, one colour.  red (color 0): i+j odd; black (color 1): i+j even.
-template <class Team>
-__device__ void half_sweep(const Team &T, const MGDev &L, int color, double omega) {
-    const int nx = L.nx, ny = L.ny, W = nx + 3;
-    const double aw = L.aw, ae = L.aw, an = L.an, as = L.an, ac = L.ac;
-    const int hw = nx / 2 + 1;
-    for (Walk2 w(T.rank(), T.size(), hw, ny + 1); w.ok(); w.next()) {
-        const int j = w.j + 1;
-        const int is = (((j + 1 + color) & 1) != 0) ? 1 : 2;
-        const int i = is + 2 * w.k;
-        if (i > nx + 1) continue;
-        const int n = i + j * W;
-        int bc = L.bc[n];
-        if (bc > 0) continue;
-        double bij = L.b[(i - 1) + (j - 1) * (nx + 1)];
-        double *u = L.u;
-        if (bc == -2) {
-            u[n] = (1.0 - omega) * u[n] + omega * (bij - an * u[n + W] - as * u[n - W] - 2.0 * ae * u[n + 1]) / ac;
-            continue;
+// A patch of a level in shared memory: the columns [ri0, ri0 + RW) and up to two runs of rows
+// (the second where the halo wraps around a periodic edge).  The row pitch is odd and the runs
+// are spaced so that i + j and the flat index q agree in parity up to a constant: a half-sweep
+// is a loop over every second q, with no rows or columns to work out.  What is to be done at a
+// node is in its mask byte:
+#define M_WALL 1     // a wall, or outside the level
+#define M_IN (-1)    // updated, and its residual counts (bcnd -1 in the tile)
+#define M_UPD 0      // updated (the same in the halo, and labels that the residual leaves out)
+#define M_NMN (-2)   // updated with the Neumann stencil
+#define M_FIX (-16)  // bcnd <= 0 but not updated (ghosts, the periodic copy, the region's rim)
+struct Patch {
+    int nx, ny;
+    int i0, i1, j0, j1;      // the tile's updatable nodes
+    int ri0, RW, RH, RP;     // RP: row pitch
+    int nA, n0, a0, b0;      // local row lr is row a0 + lr for lr < nA, b0 + lr - n0 from n0, else none
+    int clip0, clip1;        // rows that the level's edge cut off the halo, below and above
+    int par;                 // parity of i + j at q = 0
+    int wrap;                // 0: one run; 1: wrapped rows first (below row 1); 2: last; 3: every row
+    double *u, *b;
+    int8_t *m;
+    __device__ __forceinline__ int row_of(int lr) const { return lr < nA ? a0 + lr : (lr < n0 ? -1 : b0 + lr - n0); }
+    // the local row of the tile's own run
+    __device__ __forceinline__ int own(int j) const { return wrap == 2 ? j - a0 : n0 + j - b0; }
+};
+
+#define CLIP_ALL (1 << 20)   // no row of the region ever falls out of reach
+
+__device__ __forceinline__ Patch tile_patch(const MGP &P, const MGDev &L, int tile, int H, unsigned char *smem) {
+    Patch g;
+    const int nx = L.nx, ny = L.ny, TX = L.tx, TY = L.ty;
+    const int ntx = (nx + 1 + TX - 1) / TX;
+    const int tj = tile / ntx, ti = tile - tj * ntx;
+    g.nx = nx; g.ny = ny;
+    g.i0 = 1 + ti * TX;
+    g.j0 = 1 + tj * TY;
+    g.i1 = min(g.i0 + TX, nx + 2);
+    g.j1 = min(g.j0 + TY, ny + 2);
+    g.ri0 = max(g.i0 - H, 0);
+    g.RW = min(g.i1 + H, nx + 3) - g.ri0;
+    g.RP = g.RW | 1;
+    g.wrap = 0; g.nA = g.n0 = 0; g.a0 = 0;
+    g.b0 = max(g.j0 - H, 0);
+    g.RH = min(g.j1 + H, ny + 3) - g.b0;
+    g.clip0 = g.b0 - (g.j0 - H);
+    g.clip1 = g.j1 + H - (g.b0 + g.RH);
+    if (P.pbc) {
+        const bool below = g.j0 - H < 1, above = g.j1 + H - 1 > ny;
+        if (below && above) g.wrap = 3;
+        else if (below) g.wrap = g.j1 + H > ny + g.j0 - H ? 3 : 1;
+        else if (above) g.wrap = g.j1 + H - ny >= g.j0 - H ? 3 : 2;
+        if (g.wrap) { g.b0 = 0; g.clip0 = g.clip1 = 0; }
+        if (g.wrap == 3) { g.RH = ny + 3; g.clip0 = g.clip1 = CLIP_ALL; }
+        else if (g.wrap == 1) {          // rows .. ny + 1, then 0 .. (row 0 follows at the parity of ny)
+            g.a0 = ny + g.j0 - H; g.nA = ny + 2 - g.a0; g.n0 = g.nA + (ny & 1);
+            g.RH = g.n0 + g.j1 + H;
+        } else if (g.wrap == 2) {        // rows .. ny + 2, then 0 ..
+            g.a0 = g.j0 - H; g.nA = ny + 3 - g.a0; g.n0 = g.nA + ((ny + 1) & 1);
+            g.RH = g.n0 + g.j1 + H - ny;
         }
-        if (bc == 0 && j == ny + 1) continue;
-        u[n] = (1.0 - omega) * u[n] +
-               omega * (bij - aw * u[n - 1] - an * u[n + W] - as * u[n - W] - ae * u[n + 1]) / ac;
     }
+    g.par = (g.ri0 + (g.nA ? g.a0 : g.b0)) & 1;
+    g.u = (double *)smem;
+    g.b = g.u + P.cap;
+    g.m = (int8_t *)(g.b + P.cap);
+    return g;
 }
 
-// sors.f90:185-200 periodic ghost rows
-template <class Team>
-__device__ void pbc_rows(const Team &T, const MGDev &L) {
-    const int nx = L.nx, ny = L.ny, W = nx + 3;
-    for (int i = (int)T.rank(); i <= nx + 2; i += (int)T.size()) {
-        if (L.bc[i + 1 * W] <= 0) L.u[i] = L.u[i + ny * W];
-        if (L.bc[i + (ny + 1) * W] <= 0) L.u[i + (ny + 1) * W] = L.u[i + W];
-    }
-}
+// With an odd number of rows between periodic edges the nodes across the edge have the colour of
+// their neighbours, so a half-sweep's residuals are not final before the edge rows are copied:
+// such a level (only the coarsest of a deck can be one) sums them in a pass of their own.
+__device__ __forceinline__ bool odd_seam(int pbc, int ny) { return pbc && (ny & 1); }
 
-// sors.f90:338-357 L1 residual over bcnd == -1 nodes
-template <class Team>
-__device__ bool residual_l1(const Team &T, const MGDev &L, double *res) {
-    const int nx = L.nx, ny = L.ny, W = nx + 3;
-    const double aw = L.aw, ae = L.aw, an = L.an, as = L.an, ac = L.ac;
-    double acc = 0.0;
-    for (Walk2 w(T.rank(), T.size(), nx + 1, ny + 1); w.ok(); w.next()) {
-        const int t = w.flat();
-        const int n = (w.k + 1) + (w.j + 1) * W;
-        double rij = 0.0;
-        if (L.bc[n] == -1) {
-            const double *u = L.u;
-            rij = L.b[t] - (aw * u[n - 1] + an * u[n + W] + as * u[n - W] + ae * u[n + 1] + ac * u[n]);
-        }
-        acc = acc + fabs(rij);
-    }
-    return team_sum(T, acc, res);
-}
-
-// sors.f90:1-435 on one rank; returns false when a barrier failed
-template <class Team>
-__device__ bool sor_rb(const Team &T, const MGP &P, int l, int kmg, int dig, double *res_out,
-                       int *ksor_out) {
+// a whole level in CTA 0's shared memory
+__device__ __forceinline__ Patch level_patch(const MGP &P, int l, unsigned char *smem) {
     const MGDev &L = P.L[l];
-    double res = 0.0, res_s = 0.0;
-    int ksor = 0;
-    int nr = 10;
-    if (kmg == 1 && dig == 0) nr = 1000000;
-    for (int k = 1; k <= nr; k++) {
-        for (int color = 0; color < 2; color++) {
-            half_sweep(T, L, color, P.omega);
-            if (!T.sync()) return false;
-            if (P.pbc) {
-                pbc_rows(T, L);
-                if (!T.sync()) return false;
-            }
-        }
-        if (!residual_l1(T, L, &res)) return false;
-        ksor = ksor + 1;
-        if (dig == 0) {
-            if (res <= P.eps * P.alpha) break;
-        } else {
-            if (res_s > 0.0 && (res / res_s) <= 0.6) break;
-        }
-        res_s = res;
-    }
-    *res_out = res;
-    *ksor_out = ksor;
-    return true;
+    Patch g;
+    g.nx = L.nx; g.ny = L.ny;
+    g.i0 = 1; g.i1 = L.nx + 2; g.j0 = 1; g.j1 = L.ny + 2;
+    g.ri0 = 0; g.RW = L.nx + 3; g.RP = g.RW | 1; g.RH = L.ny + 3;
+    g.nA = g.n0 = 0; g.a0 = 0; g.b0 = 0;
+    g.clip0 = g.clip1 = CLIP_ALL;
+    g.par = 0;
+    g.wrap = P.pbc ? 3 : 0;
+    g.u = (double *)(smem + L.su);
+    g.b = (double *)(smem + L.sb);
+    g.m = (int8_t *)(smem + L.sm);
+    return g;
 }
 
-// mg.f90:512-547
-__device__ __forceinline__ double getres(const MGDev &L, int ir, int jr, int flag) {
-    const int W = L.nx + 3;
+// the mask byte of node (i, j) with boundary label bc; own: a row of the tile's own run
+__device__ __forceinline__ int8_t mask_of(const Patch &g, int bc, int i, int j, bool own) {
+    if (bc > 0) return M_WALL;
+    if (i < 1 || i > g.nx + 1 || j < 1 || j > g.ny + 1 || (bc == 0 && j == g.ny + 1) || i == g.ri0 || i == g.ri0 + g.RW - 1)
+        return M_FIX;
+    if (bc == -2) return M_NMN;
+    return bc == -1 && own && i >= g.i0 && i < g.i1 && j >= g.j0 && j < g.j1 ? M_IN : M_UPD;
+}
+
+// lanes per row (log2): a warp takes one, two or four rows at a time, whichever fits their width
+__device__ __forceinline__ int lanes_of(int width) { return width <= 8 ? 3 : (width <= 16 ? 4 : 5); }
+
+// t / ac, correctly rounded, for the level's fixed divisor with y = RN(1 / ac): q0 = RN(t y) is
+// within 1.5 ulp, so the first correction by the exact remainder leaves a quotient within one ulp
+// and the second rounds it correctly (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990: y correctly rounded and q within an
+// ulp make q + (t - ac q) y correctly rounded).  Five dependent operations of 8 cycles against
+// about 100 cycles of the general division, in the middle of every update's chain.  The
+// remainders are exact while t is neither tiny nor huge; outside that range (and where the host
+// found ac itself out of range: y = 0) the general division is used.
+__device__ __noinline__ double quot_general(double t, double ac) { return t / ac; }
+__device__ __forceinline__ double quot(double t, double ac, double y) {
+    const unsigned hi = (unsigned)__double2hiint(t) & 0x7fffffffu;
+    double q = t * y;
+    q = __fma_rn(__fma_rn(-ac, q, t), y, q);
+    q = __fma_rn(__fma_rn(-ac, q, t), y, q);
+    if ((hi - 0x07c00000u >= 0x70800000u && t != 0.0) || y == 0.0) q = quot_general(t, ac);
+    return q;
+}
+
+// One node's SOR update (sors.f90:80-118 / :210-248) from its loaded values; adds |r| of the
+// value before (pre) or after the update (sors.f90:338-357) to acc where it counts
+struct NodeIn { double uo, uw, ue, un, us, b; int m; };
+__device__ __forceinline__ void node_load(NodeIn &v, const double *u, const double *b, const int8_t *m, int RP) {
+    v.m = *m;
+    v.uo = u[0]; v.uw = u[-1]; v.ue = u[1]; v.un = u[RP]; v.us = u[-RP];
+    v.b = *b;
+}
+__device__ __forceinline__ void node_update(const NodeIn &v, double *u, const MGDev &L, double omega, bool pre, double &acc) {
+    if ((unsigned)(-v.m) > 4u) return;
+    const double pw = L.aw * v.uw, pn = L.an * v.un, ps = L.an * v.us, pe = L.aw * v.ue;
+    double t = v.b - pw - pn - ps - pe;
+    if (v.m == M_NMN) t = v.b - pn - ps - 2.0 * L.aw * v.ue;
+    const double unew = (1.0 - omega) * v.uo + quot(omega * t, L.ac, L.y);
+    *u = unew;
+    if (v.m == M_IN) acc += fabs(v.b - (pw + pn + ps + pe + L.ac * (pre ? v.uo : unew)));
+}
+
+// Half-sweep h of one colour by a team of T threads: red (0) is i + j odd, black (1) even.  Rows
+// within h + 1 of the region's cut edge hold values that can no longer reach the tile and are
+// left out (columns there are updated like the rest; what they hold reaches no further either).
+__device__ __forceinline__ double half_sweep(const Patch &g, const MGDev &L, int h, int color, double omega, int T) {
+    double acc = 0.0;
+    const int RP = g.RP;
+    const int lo = max(1, h + 1 - g.clip0) * RP, hi = (g.RH - max(1, h + 1 - g.clip1)) * RP;
+    int q = lo + ((lo ^ g.par ^ color ^ 1) & 1) + 2 * (int)threadIdx.x;
+    const bool pre = color == 0;
+    double *const u = g.u;
+    const double *const b = g.b;
+    const int8_t *const m = g.m;
+    for (; q + 2 * T < hi; q += 4 * T) {     // two nodes at a time: their chains overlap
+        const int p = q + 2 * T;
+        NodeIn v0, v1;
+        node_load(v0, u + q, b + q, m + q, RP);
+        node_load(v1, u + p, b + p, m + p, RP);
+        node_update(v0, u + q, L, omega, pre, acc);
+        node_update(v1, u + p, L, omega, pre, acc);
+    }
+    if (q < hi) {
+        NodeIn v0;
+        node_load(v0, u + q, b + q, m + q, RP);
+        node_update(v0, u + q, L, omega, pre, acc);
+    }
+    return acc;
+}
+
+// |r| of the last half-sweep's other colour (red), or of both, and r^2 of both, over the tile
+template <bool L2>
+__device__ __forceinline__ void last_residual(const Patch &g, const MGDev &L, double &acc, double &l2, int T, bool both = false) {
+    const double aw = L.aw, an = L.an, ac = L.ac;
+    const int RP = g.RP, step = L2 ? 1 : 2, hi = (g.RH - 1) * RP;
+    int q = RP + (L2 ? 0 : (RP ^ g.par ^ 1) & 1) + step * (int)threadIdx.x;
+#pragma unroll 2
+    for (; q < hi; q += step * T) {
+        const double *u = g.u + q;
+        const double r = g.b[q] - (aw * u[-1] + an * u[RP] + an * u[-RP] + aw * u[1] + ac * u[0]);
+        if (g.m[q] != M_IN) continue;
+        if (!L2 || both || ((q ^ g.par) & 1)) acc += fabs(r);
+        if (L2) l2 += r * r;
+    }
+}
+
+// ||b - A u_D||^2 of the tile (u_D: u with the unknowns zeroed) over bcnd == -1
+__device__ __forceinline__ double wall_norm(const Patch &g, const MGDev &L) {
+    const double aw = L.aw, an = L.an;
+    const int RP = g.RP;
+    double s = 0.0;
+    for (int q = RP + (int)threadIdx.x; q < (g.RH - 1) * RP; q += MGT) {
+        if (g.m[q] != M_IN) continue;
+        const double d = g.b[q] - ((g.m[q - 1] > 0 ? aw * g.u[q - 1] : 0.0) + (g.m[q + RP] > 0 ? an * g.u[q + RP] : 0.0) +
+                                   (g.m[q - RP] > 0 ? an * g.u[q - RP] : 0.0) + (g.m[q + 1] > 0 ? aw * g.u[q + 1] : 0.0));
+        s = s + d * d;
+    }
+    return s;
+}
+
+// sors.f90:185-200 periodic ghost rows: row 0 is row ny, row ny + 1 is row 1
+__device__ __forceinline__ void pbc_rows(const Patch &g, int T) {
+    if (!g.wrap) return;
+    const int ny = g.ny, RP = g.RP;
+    const int hi = g.wrap == 3 ? 0 : g.a0, lo = g.wrap == 3 ? 0 : g.n0;   // local rows: j - hi near ny, lo + j near 0
+    for (int k = threadIdx.x; k < g.RW; k += T) {
+        double *u = g.u + k;
+        const int8_t *m = g.m + k;
+        if (m[(lo + 1) * RP] <= 0) u[lo * RP] = u[(ny - hi) * RP];
+        if (m[(ny + 1 - hi) * RP] <= 0) u[(ny + 1 - hi) * RP] = u[(lo + 1) * RP];
+    }
+}
+
+// mg.f90:512-547 at local node q, column ir
+__device__ __forceinline__ double getres(const Patch &g, const MGDev &L, int q, int ir, int flag) {
     double aw = L.aw, ae = L.aw, an = L.an, as = L.an;
     const double ac = L.ac;
-    const int n = ir + jr * W;
-    const double *u = L.u;
-    double uij = u[n], un = u[n + W], us = u[n - W], ue = u[n + 1], uw;
+    const double *u = g.u;
+    double uij = u[q], un = u[q + g.RP], us = u[q - g.RP], ue = u[q + 1], uw;
     if (ir == 1 && flag == 1) {
         uw = 0.0;
         aw = 0;
         ae = 2.0 * ae;
     } else {
-        uw = u[n - 1];
+        uw = u[q - 1];
     }
-    double urhs = L.b[(ir - 1) + (jr - 1) * (L.nx + 1)];
-    return urhs - (aw * uw + ae * ue + an * un + as * us + ac * uij);
+    return g.b[q] - (aw * uw + ae * ue + an * un + as * us + ac * uij);
 }
 
-// r_pbc(x) of mg.f90:298-311 (zero where the reference leaves it unset)
-__device__ __forceinline__ double r_pbc(const MGDev &F, int x, int nmn) {
-    const int W = F.nx + 3, ny = F.ny;
-    bool set;
-    if (x & 1) set = F.bc[x + (ny + 1) * W] <= 0;
-    else set = (x - 1 >= 1 && F.bc[x - 1 + (ny + 1) * W] <= 0) ||
-               (x + 1 <= F.nx + 1 && F.bc[x + 1 + (ny + 1) * W] <= 0);
-    return set ? getres(F, x, ny, nmn) : 0.0;
-}
-
-// mg.f90:235-509 on one rank: full-weighting restriction of the fine residual, coarse
-// correction zeroed (the coarse mask is the precomputed injection).
-template <class Team>
-__device__ void restriction(const Team &T, const MGDev &F, const MGDev &C, int pbc, int nmn) {
-    const int nx = F.nx, ny = F.ny, W = nx + 3, nx2 = C.nx, ny2 = C.ny, W2 = nx2 + 3;
-    for (Walk2 w(T.rank(), T.size(), nx2 + 1, ny2 + 1); w.ok(); w.next()) {
-        const int t = w.flat();
-        const int i = w.k + 1, j = w.j + 1;
-        int ir = 2 * i - 1, jr = 2 * j - 1;
-        double out = 0.0;
-        if (C.bc[i + j * W2] <= 0) {
-            double r1 = 0, r2 = 0, r3 = 0, r4 = 0, r5 = 0, r6 = 0, r7 = 0, r8 = 0, r9 = 0;
-            const int8_t *bc = F.bc;
-#define FB(a, b) bc[(a) + (b) * W]
-            r9 = getres(F, ir, jr, nmn);
-            if (ir != nx + 1 && jr != ny + 1)
-                if (FB(ir + 1, jr + 1) <= 0) r1 = getres(F, ir + 1, jr + 1, nmn);
-            if (ir != nx + 1)
-                if (FB(ir + 1, jr) <= 0) r2 = getres(F, ir + 1, jr, nmn);
-            if (FB(ir + 1, jr - 1) <= 0) {
-                if (ir != nx + 1 && jr != 1) r3 = getres(F, ir + 1, jr - 1, nmn);
-                else if (jr == 1) r3 = pbc ? r_pbc(F, ir + 1, nmn) : 0.0;
-            }
-            if (FB(ir, jr - 1) <= 0) {
-                if (jr != 1) r4 = getres(F, ir, jr - 1, nmn);
-                else r4 = pbc ? r_pbc(F, ir, nmn) : 0.0;
-            }
-            if (FB(ir - 1, jr - 1) <= 0 && ir != 1) {
-                if (jr != 1) r5 = getres(F, ir - 1, jr - 1, nmn);
-                else r5 = pbc ? r_pbc(F, ir - 1, nmn) : 0.0;
-            }
-            if (FB(ir - 1, jr) <= 0)
-                if (ir != 1) r6 = getres(F, ir - 1, jr, nmn);
-            if (FB(ir - 1, jr + 1) <= 0)
-                if (ir != 1 && jr != ny + 1) r7 = getres(F, ir - 1, jr + 1, nmn);
-            if (FB(ir, jr + 1) <= 0)
-                if (jr != ny + 1) r8 = getres(F, ir, jr + 1, nmn);
-#undef FB
-            out = (4.0 * r9 + 2.0 * (r2 + r4 + r6 + r8) + r1 + r3 + r5 + r7) / 16.0;
+// The fine residual on the tile and one node around it, in place of b (the sweeps are done)
+__device__ __forceinline__ void residual_in_b(const Patch &g, const MGDev &L, int nmn) {
+    const int RP = g.RP;
+    const int c0 = max(g.i0 - 1, 1), c1 = min(g.i1 + 1, g.nx + 2);
+    const int lg = lanes_of(c1 - c0), lpr = 1 << lg;
+    const int lane = threadIdx.x & (lpr - 1), sub = threadIdx.x >> lg, nsub = MGT >> lg;
+    // r_pbc reads row ny: the wrapped run's last but one row, or any row when all are here
+    const int l0 = g.wrap == 3 ? 1 : (g.wrap == 1 ? g.ny - g.a0 : g.own(max(g.j0 - 1, 1)));
+    const int l1 = g.wrap == 3 ? g.ny + 2 : g.own(min(g.j1, g.ny + 1)) + 1;
+#pragma unroll 2
+    for (int lr = l0 + sub; lr < l1; lr += nsub) {
+        const int j = g.row_of(lr);
+        if (j < 1 || (g.wrap == 1 && lr < g.n0 && j != g.ny)) continue;
+        for (int i = c0 + lane; i < c1; i += lpr) {
+            const int q = lr * RP + i - g.ri0;
+            if (g.m[q] <= 0 || (g.wrap && j == g.ny)) g.b[q] = getres(g, L, q, i, nmn);
         }
-        C.b[t] = out;
-    }
-    const int tot2 = W2 * (ny2 + 3);
-    for (int t = (int)T.rank(); t < tot2; t += (int)T.size()) C.u[t] = 0.0;
-}
-
-// mg.f90:549-616 (each fine node has exactly one writer)
-template <class Team>
-__device__ void prolongation(const Team &T, const MGDev &C, const MGDev &F) {
-    const int W = F.nx + 3, nx2 = C.nx, ny2 = C.ny, W2 = nx2 + 3;
-    for (Walk2 w(T.rank(), T.size(), nx2 + 1, ny2 + 1); w.ok(); w.next()) {
-        const int i = w.k + 1, j = w.j + 1;
-        const double *e = C.u;
-        double r1 = e[i + j * W2], r2 = e[i + (j - 1) * W2];
-        double r3 = e[i - 1 + (j - 1) * W2], r4 = e[i - 1 + j * W2];
-        int ir = 2 * i - 1, jr = 2 * j - 1;
-        double *u = F.u;
-        const int8_t *bc = F.bc;
-        const int n = ir + jr * W;
-        if (bc[n] <= 0) u[n] = u[n] + r1;
-        if (bc[n - W] <= 0) u[n - W] = u[n - W] + (r1 + r2) / 2.0;
-        if (bc[n - W - 1] <= 0) u[n - W - 1] = u[n - W - 1] + (r1 + r2 + r3 + r4) / 4.0;
-        if (bc[n - 1] <= 0) u[n - 1] = u[n - 1] + (r1 + r4) / 2.0;
     }
 }
 
-// The part of a V-cycle on levels >= Ls, run by CTA 0: S(Ls)..R.. S*(ng-1) P.. S(Ls)
-__device__ void small_region(const MGP &P, int k, double *res, int *iter) {
-    SmallTeam T;
-    int ks;
-    const int ng = P.ng;
-    for (int l = P.Ls; l <= ng - 2; l++) {
-        sor_rb(T, P, l, k, l + 1 - ng, res, &ks);
-        iter[l] += ks;
-        restriction(T, P.L[l], P.L[l + 1], P.pbc, P.nmn);
-        __syncthreads();
+// mg.f90:235-509 on one rank: full-weighting restriction of the fine residual (held in g.b) at
+// the coarse nodes whose fine centre lies in the tile; put(i, j, value) stores it (the coarse
+// mask is the precomputed injection, its value read by mask(i, j))
+template <class Mask, class Put>
+__device__ __forceinline__ void restriction(const Patch &g, int pbc, Mask mask, Put put) {
+    const int nx = g.nx, ny = g.ny, RP = g.RP;
+    const int ic0 = (g.i0 + 2) / 2, ic1 = g.i1 / 2 + 1, jc0 = (g.j0 + 2) / 2, jc1 = g.j1 / 2 + 1;
+    const int lg = lanes_of(ic1 - ic0), lpr = 1 << lg;
+    const int lane = threadIdx.x & (lpr - 1), sub = threadIdx.x >> lg, nsub = MGT >> lg;
+    const int lny = g.wrap == 3 ? ny : ny - g.a0, lny1 = lny + 1;   // local rows of ny and ny + 1 (periodic)
+    // r_pbc(x) of mg.f90:298-311 (zero where the reference leaves it unset)
+    auto rpbc = [&](int x) {
+        const int8_t *t = g.m + lny1 * RP - g.ri0;
+        bool set;
+        if (x & 1) set = t[x] <= 0;
+        else set = (x - 1 >= 1 && t[x - 1] <= 0) || (x + 1 <= nx + 1 && t[x + 1] <= 0);
+        return set ? g.b[lny * RP + x - g.ri0] : 0.0;
+    };
+    for (int j = jc0 + sub; j < jc1; j += nsub)
+        for (int i = ic0 + lane; i < ic1; i += lpr) {
+            const int ir = 2 * i - 1, jr = 2 * j - 1;
+            double out = 0.0;
+            if (mask(i, j) <= 0) {
+                const int q = g.own(jr) * RP + ir - g.ri0;
+                const double *r = g.b + q;
+                const int8_t *m = g.m + q;
+                double r1 = 0, r2 = 0, r3 = 0, r4 = 0, r5 = 0, r6 = 0, r7 = 0, r8 = 0;
+                const double r9 = r[0];
+                if (ir != nx + 1 && jr != ny + 1)
+                    if (m[1 + RP] <= 0) r1 = r[1 + RP];
+                if (ir != nx + 1)
+                    if (m[1] <= 0) r2 = r[1];
+                if (m[1 - RP] <= 0) {
+                    if (ir != nx + 1 && jr != 1) r3 = r[1 - RP];
+                    else if (jr == 1) r3 = pbc ? rpbc(ir + 1) : 0.0;
+                }
+                if (m[-RP] <= 0) {
+                    if (jr != 1) r4 = r[-RP];
+                    else r4 = pbc ? rpbc(ir) : 0.0;
+                }
+                if (m[-1 - RP] <= 0 && ir != 1) {
+                    if (jr != 1) r5 = r[-1 - RP];
+                    else r5 = pbc ? rpbc(ir - 1) : 0.0;
+                }
+                if (m[-1] <= 0)
+                    if (ir != 1) r6 = r[-1];
+                if (m[-1 + RP] <= 0)
+                    if (ir != 1 && jr != ny + 1) r7 = r[-1 + RP];
+                if (m[RP] <= 0)
+                    if (jr != ny + 1) r8 = r[RP];
+                out = (4.0 * r9 + 2.0 * (r2 + r4 + r6 + r8) + r1 + r3 + r5 + r7) / 16.0;
+            }
+            put(i, j, out);
+        }
+}
+
+// mg.f90:549-616 at fine node (i, j), 0 <= i <= nx + 1, 0 <= j <= ny + 1: u plus the coarse
+// correction e (each fine node has one coarse node whose stencil holds it; W2: e's row length)
+__device__ __forceinline__ double prolonged(double u, const double *e, int W2, int i, int j) {
+    const double *p = e + (i + 2) / 2 + ((j + 2) / 2) * W2;
+    const double r1 = p[0];
+    if (i & 1) {
+        if (j & 1) return u + r1;
+        return u + (r1 + p[-W2]) / 2.0;
     }
-    sor_rb(T, P, ng - 1, k, 0, res, &ks);
-    iter[ng - 1] += ks;
-    if (ng - 1 > P.Ls) {
-        prolongation(T, P.L[ng - 1], P.L[ng - 2]);
-        __syncthreads();
+    if (j & 1) return u + (r1 + p[-1]) / 2.0;
+    return u + (r1 + p[-W2] + p[-1 - W2] + p[-1]) / 4.0;
+}
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = v + __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// one double global -> shared without a register round trip
+__device__ __forceinline__ void cp_async8(double *dst, const double *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+struct MGShared {
+    Patch g;                        // the patch being worked on
+    double acc[MG_NR][MGW];         // a pass's sums per warp
+    double tot[MG_NR];
+    double red[MGW], res;           // CTA 0's sums and last residual
+    int pred[2][LEPIC_MAXLEV];      // sweeps a stage took last time, down and up
+    int iter[LEPIC_MAXLEV];
+};
+
+#define SRC_ZERO 0        // a correction: starts from zeros
+#define SRC_U 1           // the level's current buffer
+#define SRC_UP 2          // ... plus the prolongation of the next level's
+
+__device__ __forceinline__ double *buf_of(const MGDev &L, int which) { return which ? L.u2 : L.u; }
+
+// the barrier of the CTA's first T threads (T a multiple of 32)
+__device__ __forceinline__ void team_sync(int T) {
+    if (T == 32) __syncwarp();
+    else asm volatile("bar.sync 1, %0;" :: "r"(T) : "memory");
+}
+
+// K sweeps of the patch S.g by a team of T threads, each sweep's sum of |r| added to S.acc (and r^2
+// after the last one with l2).  A black half-sweep adds the residuals of its own nodes (their red
+// neighbours are final), the next red one those of the red nodes before it updates them.
+__device__ __forceinline__ void sweeps(const MGP &P, MGShared &S, const MGDev &L, int K, int T, bool l2) {
+    const Patch &g = S.g;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool seam = odd_seam(P.pbc, L.ny);
+    double a0 = 0.0, unused = 0.0;
+    for (int h = 0; h < 2 * K; h++) {
+        const int color = h & 1;
+        double a = half_sweep(g, L, h, color, P.omega, T);
+        team_sync(T);
+        if (P.pbc) { pbc_rows(g, T); team_sync(T); }
+        if (seam) {
+            a = 0.0;
+            if (color) { last_residual<true>(g, L, a, unused, T, true); team_sync(T); }
+        }
+        if (color) {
+            a0 = a;
+        } else if (h) {
+            a0 = warp_sum(a0 + a);
+            if (lane == 0) S.acc[(h >> 1) - 1][warp] += a0;
+        }
     }
-    for (int l = ng - 2; l >= P.Ls; l--) {
-        sor_rb(T, P, l, k, ng - l - 1, res, &ks);
-        iter[l] += ks;
-        if (l > P.Ls) {
-            prolongation(T, P.L[l], P.L[l - 1]);
+    double q2 = 0.0;
+    if (l2) last_residual<true>(g, L, seam ? unused : a0, q2, T);
+    else if (!seam) last_residual<false>(g, L, a0, q2, T);
+    a0 = warp_sum(a0);
+    if (lane == 0) S.acc[K - 1][warp] += a0;
+    if (l2) {
+        q2 = warp_sum(q2);
+        if (lane == 0) S.acc[MG_KMAX][warp] += q2;
+    }
+}
+
+// One pass over level l: K sweeps of every tile from buffer `cur` into the other one.  Sums of
+// the pass into S.acc (summed over this CTA's tiles).
+__device__ __forceinline__ void tile_pass(const MGP &P, MGShared &S, int l, int cur, int src, int ccur, int K, bool restr, bool l2,
+                          bool bb, unsigned char *smem) {
+    const MGDev &L = P.L[l];
+    const Patch &g = S.g;              // in shared memory: read where needed, no registers held
+    const int nx = L.nx, ny = L.ny, W = nx + 3;
+    const double *uin = buf_of(L, cur);
+    double *uout = buf_of(L, cur ^ 1);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane < MG_NSUM) S.acc[lane][warp] = 0.0;
+    const int ntiles = ((nx + 1 + L.tx - 1) / L.tx) * ((ny + 1 + L.ty - 1) / L.ty);
+    const int first = P.Ls < P.ng ? 1 : 0;       // CTA 0 keeps its shared memory for the coarse levels
+    const int H = 2 * K + (restr ? 2 : 1);
+    for (int tile = (int)blockIdx.x - first; tile >= 0 && tile < ntiles; tile += (int)gridDim.x - first) {
+        if (threadIdx.x == 0) S.g = tile_patch(P, L, tile, H, smem);
+        __syncthreads();
+        const int lg = lanes_of(g.RP), lpr = 1 << lg;
+        const int ln = threadIdx.x & (lpr - 1), sub = threadIdx.x >> lg, nsub = MGT >> lg;
+        for (int lr = sub; lr < g.RH; lr += nsub) {
+            const int j = g.row_of(lr);
+            const bool jb = j >= 1 && j <= ny + 1;
+            for (int k = ln; k < g.RW; k += lpr) {
+                const int i = g.ri0 + k, q = lr * g.RP + k;
+                if (jb && i >= 1 && i <= nx + 1)
+                    cp_async8(g.b + q, L.b + (i - 1) + (long long)(j - 1) * (nx + 1));
+                else
+                    g.b[q] = 0.0;
+                if (src == SRC_ZERO || j < 0) g.u[q] = 0.0;
+                else cp_async8(g.u + q, uin + i + (long long)j * W);
+            }
+        }
+        // the mask bytes of four rows at a time, so that their loads overlap
+        for (int lr0 = sub; lr0 < g.RH; lr0 += 4 * nsub)
+            for (int k = ln; k < g.RP; k += lpr) {
+                int bc[4];
+#pragma unroll
+                for (int v = 0; v < 4; v++) {
+                    const int lr = lr0 + v * nsub;
+                    const int j = lr < g.RH ? g.row_of(lr) : -1;
+                    bc[v] = j >= 0 && k < g.RW ? (int)__ldg(L.bc + g.ri0 + k + (long long)j * W) : 1;
+                }
+#pragma unroll
+                for (int v = 0; v < 4; v++) {
+                    const int lr = lr0 + v * nsub;
+                    if (lr < g.RH)
+                        g.m[lr * g.RP + k] = mask_of(g, bc[v], g.ri0 + k, g.row_of(lr), g.wrap == 2 ? lr < g.nA : lr >= g.n0);
+                }
+            }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        if (src == SRC_UP) {
+            const MGDev &C = P.L[l + 1];
+            const double *e = buf_of(C, ccur);
+            const int W2 = C.nx + 3;
+#pragma unroll 2
+            for (int lr = sub; lr < g.RH; lr += nsub) {
+                const int j = g.row_of(lr);
+                if (j < 0 || j > ny + 1) continue;
+                for (int k = ln; k < g.RW; k += lpr) {
+                    const int i = g.ri0 + k, q = lr * g.RP + k;
+                    if (i <= nx + 1 && g.m[q] <= 0) g.u[q] = prolonged(g.u[q], e, W2, i, j);
+                }
+            }
             __syncthreads();
         }
+        if (bb) {
+            const double t = warp_sum(wall_norm(g, L));
+            if (lane == 0) S.acc[MG_KMAX + 1][warp] += t;
+        }
+        sweeps(P, S, L, K, MGT, l2);
+        // the tile, and for a tile on the border the ghost nodes beside it: the tiles together
+        // write every node of the level exactly once
+        {
+            const int wi0 = g.i0 == 1 ? 0 : g.i0, wj0 = g.j0 == 1 ? 0 : g.j0;
+            const int wi1 = g.i1 == nx + 2 ? nx + 3 : g.i1, wj1 = g.j1 == ny + 2 ? ny + 3 : g.j1;
+            for (int j = wj0 + sub; j < wj1; j += nsub)
+                for (int i = wi0 + ln; i < wi1; i += lpr)
+                    uout[i + (long long)j * W] = g.u[g.own(j) * g.RP + i - g.ri0];
+        }
+        if (restr) {
+            const MGDev &C = P.L[l + 1];
+            __syncthreads();           // the residual sums have read b
+            residual_in_b(g, L, P.nmn);
+            __syncthreads();
+            restriction(g, P.pbc, [&](int i, int j) { return (int)__ldg(C.bc + i + (long long)j * (C.nx + 3)); },
+                        [&](int i, int j, double v) { C.b[(i - 1) + (long long)(j - 1) * (C.nx + 1)] = v; });
+        }
+        __syncthreads();
     }
 }
 
-// mg.f90:85-225 -- one V-cycle; *res is the L1 residual of the last finest-level sweep
-__device__ bool vcycle(const MGP &P, int k, double *res, int *iter) {
-    BigTeam B{P.cnt, P.partials, P.bar_extra};
-    const int ng = P.ng, Ls = P.Ls;
-    int ks;
-    for (int l = 0; l < Ls && l <= ng - 2; l++) {
-        if (!sor_rb(B, P, l, k, l + 1 - ng, res, &ks)) return false;
-        iter[l] += ks;
-        restriction(B, P.L[l], P.L[l + 1], P.pbc, P.nmn);
-        if (!B.sync()) return false;
+// every CTA's S.acc summed in a fixed order into S.tot, behind the grid barrier that also ends
+// the pass; the sums alternate between the halves of `partials`, so that a CTA that runs ahead
+// writes none of the slots still being read
+__device__ bool pass_sums(const MGP &P, MGShared &S, unsigned *phase) {
+    __syncthreads();
+    double *part = P.partials + (*phase & 1) * MG_NSUM * gridDim.x;
+    *phase += 1;
+    if (threadIdx.x < MG_NSUM) {
+        double a = 0.0;
+#pragma unroll
+        for (int w = 0; w < MGW; w++) a = a + S.acc[threadIdx.x][w];
+        part[threadIdx.x * gridDim.x + blockIdx.x] = a;
     }
-    int top;
-    if (Ls <= ng - 1) {
-        if (blockIdx.x == 0) {
-            double r = 0.0;
-            small_region(P, k, &r, iter);
-            if (threadIdx.x == 0) P.cnt->mg_res_l1 = r;
-        }
-        if (!B.sync()) return false;
-        *res = ((volatile double *)&P.cnt->mg_res_l1)[0];
-        top = Ls;
-    } else {
-        if (!sor_rb(B, P, ng - 1, k, 0, res, &ks)) return false;
-        iter[ng - 1] += ks;
-        top = ng - 1;
+    if (!grid_barrier(P.cnt, gridDim.x + P.bar_extra)) return false;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < MG_NSUM) {
+        double a = 0.0;
+        for (int i = lane; i < (int)gridDim.x; i += 32) a = a + __ldcg(part + warp * gridDim.x + i);
+        a = warp_sum(a);
+        if (lane == 0) S.tot[warp] = a;
     }
-    if (top >= 1) {
-        prolongation(B, P.L[top], P.L[top - 1]);
-        if (!B.sync()) return false;
-    }
-    for (int l = top - 1; l >= 0; l--) {
-        if (!sor_rb(B, P, l, k, ng - l - 1, res, &ks)) return false;
-        iter[l] += ks;
-        if (l >= 1) {
-            prolongation(B, P.L[l], P.L[l - 1]);
-            if (!B.sync()) return false;
-        }
-    }
+    __syncthreads();
     return true;
 }
 
-// ||b - A u||_2^2 and ||b - A u_D||_2^2 (u_D: u with the unknowns zeroed) over bcnd == -1
-template <class Team>
-__device__ bool l2_norms(const Team &T, const MGDev &L, double *rr, double *bb) {
-    const int nx = L.nx, ny = L.ny, W = nx + 3;
-    const double aw = L.aw, ae = L.aw, an = L.an, as = L.an, ac = L.ac;
-    double a = 0.0, b = 0.0;
-    for (Walk2 w(T.rank(), T.size(), nx + 1, ny + 1); w.ok(); w.next()) {
-        const int t = w.flat();
-        const int n = (w.k + 1) + (w.j + 1) * W;
-        if (L.bc[n] != -1) continue;
-        const double *u = L.u;
-        const int8_t *bc = L.bc;
-        double r = L.b[t] - (aw * u[n - 1] + an * u[n + W] + as * u[n - W] + ae * u[n + 1] + ac * u[n]);
-        double d = L.b[t] - ((bc[n - 1] > 0 ? aw * u[n - 1] : 0.0) + (bc[n + W] > 0 ? an * u[n + W] : 0.0) +
-                             (bc[n - W] > 0 ? as * u[n - W] : 0.0) + (bc[n + 1] > 0 ? ae * u[n + 1] : 0.0));
-        a = a + r * r;
-        b = b + d * d;
+// sors.f90:1-435 on one rank for a level of the tile passes; false when a barrier failed.  dir: 0
+// down, 1 up (where the predicted sweep count is kept)
+__device__ bool sor_big(const MGP &P, MGShared &S, int l, int kmg, int dig, int dir, int src, bool restr, bool l2,
+                        bool bb, unsigned &curs, unsigned *phase, unsigned char *smem, double *res_out, double *bb_out) {
+    double res = 0.0, res_s = 0.0;
+    const int nr = kmg == 1 && dig == 0 ? 1000000 : MG_NR;
+    const int want = S.pred[dir][l];
+    int done = 0;
+    for (;;) {
+        // more than MG_KMAX sweeps are split evenly; past the prediction two, then MG_KMAX
+        int K = done ? MG_KMAX : 2;
+        if (done < want) {
+            const int left = want - done, parts = (left + MG_KMAX - 1) / MG_KMAX;
+            K = (left + parts - 1) / parts;
+        }
+        K = min(K, nr - done);
+        const int cur = (curs >> l) & 1, ccur = (curs >> (l + 1)) & 1;
+        tile_pass(P, S, l, cur, src, ccur, K, restr, l2, bb, smem);
+        if (!pass_sums(P, S, phase)) return false;
+        if (bb) *bb_out = S.tot[MG_KMAX + 1];
+        bb = false;
+        bool stop = false;
+        int q = 0;
+        for (; q < K && !stop; q++) {
+            res = S.tot[q];
+            if (dig == 0) stop = res <= P.eps * P.alpha;
+            else stop = res_s > 0.0 && (res / res_s) <= 0.6;
+            if (!stop) {
+                res_s = res;
+                stop = done + q + 1 == nr;
+            }
+        }
+        if (stop && q < K) {          // the reference stops earlier: the pass again, that far only
+            __syncthreads();
+            tile_pass(P, S, l, cur, src, ccur, q, restr, l2, false, smem);
+            if (!pass_sums(P, S, phase)) return false;
+        }
+        curs ^= 1u << l;
+        done += q;
+        src = SRC_U;
+        if (stop) break;
     }
-    if (!team_sum(T, a, rr)) return false;
-    return team_sum(T, b, bb);
+    __syncthreads();
+    if (threadIdx.x == 0) { S.pred[dir][l] = done; S.iter[l] += done; }
+    __syncthreads();
+    *res_out = res;
+    return true;
+}
+
+// sor_big's decisions for a level in CTA 0's shared memory: the predicted number of sweeps (else
+// two, then the rest) from a copy kept in the level's global buffer, their residuals summed
+// together, and the sweeps taken again from the copy where the reference stops earlier.  The
+// stages take two sweeps or all ten, so a prediction rarely fails.
+__device__ void sor_small(const MGP &P, MGShared &S, int l, int kmg, int dig, int dir, unsigned char *smem, double *res_out) {
+    const Patch &g = S.g;
+    const MGDev &L = P.L[l];
+    if (threadIdx.x == 0) S.g = level_patch(P, l, smem);
+    __syncthreads();
+    // only as many warps as the level has nodes of one colour: idle warps cost issue slots and a
+    // slower barrier
+    const int T = min(MGT, (g.RP * g.RH / 2 + 31) & ~31);
+    if ((int)threadIdx.x < T) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = T >> 5;
+        const int nn = g.RP * g.RH;
+        double *keep = L.u2;
+        double res = 0.0, res_s = 0.0;
+        const int nr = kmg == 1 && dig == 0 ? 1000000 : MG_NR;
+        const int want = S.pred[dir][l];
+        int done = 0;
+        bool stop = false;
+        while (!stop) {
+            const int K = min(min(done < want ? want - done : (done ? 8 : 2), MG_NR), nr - done);
+            const bool sure = done == 0 && dig != 0 && K <= 2;     // the second sweep is always taken
+            if (!sure)
+                for (int t = threadIdx.x; t < nn; t += T) keep[t] = g.u[t];
+            if (lane < MG_NR) S.acc[lane][warp] = 0.0;
+            team_sync(T);
+            sweeps(P, S, L, K, T, false);
+            team_sync(T);
+            // every warp adds up the sums it needs by itself: lane q takes sweep q's
+            double tot = 0.0;
+            if (lane < K)
+                for (int w = 0; w < nw; w++) tot = tot + S.acc[lane][w];
+            int q = 0;
+            for (; q < K && !stop; q++) {
+                res = __shfl_sync(0xffffffffu, tot, q);
+                if (dig == 0) stop = res <= P.eps * P.alpha;
+                else stop = res_s > 0.0 && (res / res_s) <= 0.6;
+                if (!stop) {
+                    res_s = res;
+                    stop = done + q + 1 == nr;
+                }
+            }
+            if (stop && q < K) {
+                team_sync(T);
+                for (int t = threadIdx.x; t < nn; t += T) g.u[t] = keep[t];
+                team_sync(T);
+                sweeps(P, S, L, q, T, false);
+            }
+            done += q;
+            team_sync(T);
+        }
+        if (threadIdx.x == 0) { S.pred[dir][l] = done; S.iter[l] += done; S.res = res; }
+    }
+    __syncthreads();
+    *res_out = S.res;
+}
+
+// a CTA-wide sum for CTA 0's own levels, outside the sweeps
+__device__ double cta_sum(MGShared &S, double v) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();
+    v = warp_sum(v);
+    if (lane == 0) S.red[warp] = v;
+    __syncthreads();
+    double a = 0.0;
+#pragma unroll
+    for (int w = 0; w < MGW; w++) a = a + S.red[w];
+    __syncthreads();
+    return a;
+}
+
+// The part of a V-cycle on levels >= Ls, run by CTA 0: S(Ls)..R.. S*(ng-1) P.. S(Ls)
+__device__ void small_region(const MGP &P, MGShared &S, int k, unsigned char *smem, double *res) {
+    const int ng = P.ng, Ls = P.Ls;
+    if (Ls > 0) {     // the restricted residual of level Ls - 1 in, its correction from zeros
+        const MGDev &L = P.L[Ls];
+        const Patch g = level_patch(P, Ls, smem);
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll 2
+        for (int j = warp; j < L.ny + 3; j += MGW)
+            for (int i = lane; i < L.nx + 3; i += 32) {
+                g.u[i + j * g.RP] = 0.0;
+                if (i >= 1 && i <= L.nx + 1 && j >= 1 && j <= L.ny + 1)
+                    g.b[i + j * g.RP] = __ldcg(L.b + (i - 1) + (j - 1) * (L.nx + 1));
+            }
+        __syncthreads();
+    }
+    for (int l = Ls; l <= ng - 2; l++) {
+        sor_small(P, S, l, k, l + 1 - ng, 0, smem, res);
+        const Patch g = level_patch(P, l, smem), c = level_patch(P, l + 1, smem);
+        // b holds the level's right-hand side, which the way up needs again: the residual goes to
+        // the coarse patch's u and b by way of registers, nine values per coarse node
+        const MGDev &L = P.L[l];
+        for (int t = threadIdx.x; t < c.RP * c.RH; t += MGT) c.u[t] = 0.0;
+        {
+            const int nx = g.nx, ny = g.ny, RP = g.RP;
+            const int lg = lanes_of(c.nx + 1), lpr = 1 << lg;
+            const int lane = threadIdx.x & (lpr - 1), sub = threadIdx.x >> lg, nsub = MGT >> lg;
+            auto R = [&](int q, int x) { return getres(g, L, q, x, P.nmn); };
+            auto rpbc = [&](int x) {
+                const int8_t *t = g.m + (ny + 1) * RP;
+                bool set;
+                if (x & 1) set = t[x] <= 0;
+                else set = (x - 1 >= 1 && t[x - 1] <= 0) || (x + 1 <= nx + 1 && t[x + 1] <= 0);
+                return set ? R(ny * RP + x, x) : 0.0;
+            };
+            for (int j = 1 + sub; j <= c.ny + 1; j += nsub)
+                for (int i = 1 + lane; i <= c.nx + 1; i += lpr) {
+                    const int ir = 2 * i - 1, jr = 2 * j - 1, q = ir + jr * RP;
+                    double out = 0.0;
+                    if (c.m[i + j * c.RP] <= 0) {
+                        const int8_t *m = g.m + q;
+                        double r1 = 0, r2 = 0, r3 = 0, r4 = 0, r5 = 0, r6 = 0, r7 = 0, r8 = 0;
+                        const double r9 = R(q, ir);
+                        if (ir != nx + 1 && jr != ny + 1)
+                            if (m[1 + RP] <= 0) r1 = R(q + 1 + RP, ir + 1);
+                        if (ir != nx + 1)
+                            if (m[1] <= 0) r2 = R(q + 1, ir + 1);
+                        if (m[1 - RP] <= 0) {
+                            if (ir != nx + 1 && jr != 1) r3 = R(q + 1 - RP, ir + 1);
+                            else if (jr == 1) r3 = P.pbc ? rpbc(ir + 1) : 0.0;
+                        }
+                        if (m[-RP] <= 0) {
+                            if (jr != 1) r4 = R(q - RP, ir);
+                            else r4 = P.pbc ? rpbc(ir) : 0.0;
+                        }
+                        if (m[-1 - RP] <= 0 && ir != 1) {
+                            if (jr != 1) r5 = R(q - 1 - RP, ir - 1);
+                            else r5 = P.pbc ? rpbc(ir - 1) : 0.0;
+                        }
+                        if (m[-1] <= 0)
+                            if (ir != 1) r6 = R(q - 1, ir - 1);
+                        if (m[-1 + RP] <= 0)
+                            if (ir != 1 && jr != ny + 1) r7 = R(q - 1 + RP, ir - 1);
+                        if (m[RP] <= 0)
+                            if (jr != ny + 1) r8 = R(q + RP, ir);
+                        out = (4.0 * r9 + 2.0 * (r2 + r4 + r6 + r8) + r1 + r3 + r5 + r7) / 16.0;
+                    }
+                    c.b[i + j * c.RP] = out;
+                }
+        }
+        __syncthreads();
+    }
+    sor_small(P, S, ng - 1, k, 0, 0, smem, res);
+    for (int l = ng - 2; l >= Ls; l--) {
+        const Patch g = level_patch(P, l, smem), c = level_patch(P, l + 1, smem);
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        for (int j = warp; j <= g.ny + 1; j += MGW)
+            for (int i = lane; i <= g.nx + 1; i += 32) {
+                const int q = i + j * g.RP;
+                if (g.m[q] <= 0) g.u[q] = prolonged(g.u[q], c.u, c.RP, i, j);
+            }
+        __syncthreads();
+        sor_small(P, S, l, k, ng - l - 1, 1, smem, res);
+    }
+    if (Ls > 0) {     // the correction out
+        const MGDev &L = P.L[Ls];
+        const Patch g = level_patch(P, Ls, smem);
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        for (int j = warp; j < L.ny + 3; j += MGW)
+            for (int i = lane; i < L.nx + 3; i += 32) L.u[i + j * (L.nx + 3)] = g.u[i + j * g.RP];
+    }
 }
 
 // iterative_solver.f90:18-66.  mode 0: stop on the reference's normalised L1 residual;
 // mode 2: same cycles, stop on ||b-Au||_2/||b-Au_D||_2 <= eps.
-__global__ void __launch_bounds__(MG_THREADS) k_mg_solve(MGP P) {
-    BigTeam B{P.cnt, P.partials, P.bar_extra};
-    int iter[LEPIC_MAXLEV];
-    for (int i = 0; i < LEPIC_MAXLEV; i++) iter[i] = 0;
+__global__ void __launch_bounds__(MGT, 2) k_mg_solve(const __grid_constant__ MGP P) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ MGShared S;
+    const int ng = P.ng, Ls = P.Ls;
     double res = 0.0, res_s = 0.0, rr = 0.0, bb = 0.0;
+    unsigned curs = 0, phase = 0;       // each level's current buffer; sums taken so far
+    for (int t = threadIdx.x; t < LEPIC_MAXLEV; t += MGT) { S.pred[0][t] = S.pred[1][t] = 0; S.iter[t] = 0; }
+    const bool small = Ls < ng && blockIdx.x == 0;
+    if (small) {                        // the coarse levels' masks (and level 0's u and b when it is one of them)
+        for (int l = Ls; l < ng; l++) {
+            const Patch g = level_patch(P, l, smem);
+            const MGDev &L = P.L[l];
+            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+            for (int j = warp; j < g.RH; j += MGW)
+                for (int i = lane; i < g.RP; i += 32) {
+                    const int q = i + j * g.RP;
+                    const int n = i + j * g.RW;
+                    g.m[q] = i < g.RW ? mask_of(g, L.bc[n], i, j, true) : M_WALL;
+                    g.u[q] = l == 0 && i < g.RW ? L.u[n] : 0.0;
+                    g.b[q] = l == 0 && i >= 1 && i <= L.nx + 1 && j >= 1 && j <= L.ny + 1 ? L.b[(i - 1) + (j - 1) * (L.nx + 1)] : 0.0;
+                }
+        }
+    }
+    __syncthreads();
+    if (Ls == 0) {                      // one CTA holds the whole problem
+        if (!grid_barrier(P.cnt, gridDim.x + P.bar_extra)) return;
+        bb = cta_sum(S, wall_norm(level_patch(P, 0, smem), P.L[0]));
+    }
     int k = 1;
-    if (P.mode == 2 && !l2_norms(B, P.L[0], &rr, &bb)) return;
-    const double b0 = sqrt(bb);
-    bool conv = false;
+    bool conv = false, diverged = false;
     for (;;) {
-        if (!vcycle(P, k, &res, iter)) return;
-        res = res / P.alpha;
-        bool diverged = false;
-        if (k == 1) res_s = res;
-        else if (fabs(res / res_s) > 10.0) diverged = true;
-        if (diverged) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) set_err(P.cnt, LERR_DIVERGED, 500);
-            return; // every CTA takes the same decision
+        // mg.f90:85-225 -- one V-cycle; res is the L1 residual of the last finest-level sweep
+        for (int l = 0; l < Ls && l <= ng - 2; l++) {
+            const int src = l == 0 ? SRC_U : SRC_ZERO;
+            if (!sor_big(P, S, l, k, l + 1 - ng, 0, src, true, false, k == 1 && l == 0, curs, &phase, smem, &res, &bb)) return;
         }
-        if (P.mode == 2) {
-            if (!l2_norms(B, P.L[0], &rr, &bb)) return;
-            conv = sqrt(rr) <= P.eps * b0;
+        int top = Ls;
+        if (Ls < ng) {
+            curs &= ~(1u << Ls);        // the correction of level Ls is left in its first buffer
+            if (small) {
+                __syncthreads();
+                small_region(P, S, k, smem, &res);
+            }
+            if (Ls > 0 && !grid_barrier(P.cnt, gridDim.x + P.bar_extra)) return;
         } else {
-            conv = res <= P.eps;
+            const int l = ng - 1;
+            if (!sor_big(P, S, l, k, 0, 0, l == 0 ? SRC_U : SRC_ZERO, false, l == 0, k == 1 && l == 0, curs, &phase, smem,
+                         &res, &bb)) return;
+            top = ng - 1;
         }
+        for (int l = top - 1; l >= 0; l--)
+            if (!sor_big(P, S, l, k, ng - l - 1, 1, SRC_UP, false, l == 0, false, curs, &phase, smem, &res, &bb)) return;
+        if (Ls == 0) {
+            double a = 0.0, q2 = 0.0;
+            last_residual<true>(level_patch(P, 0, smem), P.L[0], a, q2, MGT);
+            rr = cta_sum(S, q2);
+        } else {
+            rr = S.tot[MG_KMAX];
+        }
+        res = res / P.alpha;
+        if (k == 1) res_s = res;
+        else if (fabs(res / res_s) > 10.0) { diverged = true; break; }
+        if (P.mode == 2) conv = sqrt(rr) <= P.eps * sqrt(bb);
+        else conv = res <= P.eps;
         if (conv || k == P.ncycl) break;
         k = k + 1;
     }
-    if (!l2_norms(B, P.L[0], &rr, &bb)) return;
+    // the potential into phi
+    if (Ls == 0) {
+        const Patch g = level_patch(P, 0, smem);
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        for (int j = warp; j < g.RH; j += MGW)
+            for (int i = lane; i < g.RW; i += 32) P.L[0].u[i + j * g.RW] = g.u[i + j * g.RP];
+    } else if (curs & 1u) {
+        const long long nn = (long long)(P.L[0].nx + 3) * (P.L[0].ny + 3);
+        for (long long t = blockIdx.x * (long long)MGT + threadIdx.x; t < nn; t += (long long)gridDim.x * MGT)
+            P.L[0].u[t] = P.L[0].u2[t];
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (diverged) { set_err(P.cnt, LERR_DIVERGED, 500); return; }
         // ncycl cycles without reaching eps: the reference goes on with this potential
         // (iterative_solver.f90:56); the call reports it and phi holds the last cycle's result
         if (!conv) set_err(P.cnt, LERR_NOTCONV, 501);
         double ktot = 0.0;
-        for (int i = 1; i <= P.ng; i++) ktot = ktot + (double)iter[i - 1] / pow(2.0, 2 * (i - 1));
+        for (int i = 1; i <= ng; i++) ktot = ktot + (double)S.iter[i - 1] / pow(2.0, 2 * (i - 1));
         P.cnt->mg_cycles = k;
-        P.cnt->mg_sweeps_fine = iter[0];
+        P.cnt->mg_sweeps_fine = S.iter[0];
         P.cnt->mg_res_l1 = res;
         P.cnt->mg_ktot = ktot;
         P.cnt->mg_res_l2 = sqrt(rr);
@@ -358,20 +866,9 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_solve(MGP P) {
     }
 }
 
-// Stats only: the L1 and L2 residuals of the current phi.
-__global__ void __launch_bounds__(MG_THREADS) k_mg_stats(MGP P) {
-    BigTeam B{P.cnt, P.partials, P.bar_extra};
-    double res = 0.0, rr = 0.0, bb = 0.0;
-    if (!residual_l1(B, P.L[0], &res)) return;
-    if (!l2_norms(B, P.L[0], &rr, &bb)) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        P.cnt->mg_res_l1 = res / P.alpha;
-        P.cnt->mg_res_l2 = sqrt(rr);
-        P.cnt->mg_b_l2 = sqrt(bb);
-    }
-}
-
 // ---------------------------------------------------------------------------------------
+#define MG_SMEM (110 * 1024)   // dynamic shared memory per CTA (two per SM)
+
 static MGP mg_params(lepic_ctx *c, double eps, int mode) {
     MGP P;
     memset(&P, 0, sizeof(P));
@@ -379,18 +876,46 @@ static MGP mg_params(lepic_ctx *c, double eps, int mode) {
     for (int l = 0; l < c->nlev; l++) {
         MGLevel &a = c->lev[l];
         MGDev &d = P.L[l];
-        d.nx = a.nx; d.ny = a.ny; d.hx = a.hx; d.hy = a.hy;
+        d.nx = a.nx; d.ny = a.ny;
         d.aw = eps0 / (a.hx * a.hx);
         d.an = eps0 / (a.hy * a.hy);
         d.ac = -(d.an + d.an + d.aw + d.aw);
+        d.y = fabs(d.ac) > 1e-30 && fabs(d.ac) < 1e30 ? 1.0 / d.ac : 0.0;
         d.u = a.u; d.b = a.b; d.bc = a.bc;
+        d.u2 = l == 0 ? c->cg_ap : a.u2;
     }
     P.ng = c->nlev;
+    // the CTA-0 part: the coarsest levels, as long as each has at most small_nodes nodes and
+    // they fit in shared memory together
     const long long small_nodes = c->opt.mg_small_nodes;
-    int Ls = c->nlev;
-    for (int l = 0; l < c->nlev; l++)
-        if ((long long)(c->lev[l].nx + 1) * (c->lev[l].ny + 1) <= small_nodes) { Ls = l; break; }
-    P.Ls = Ls;
+    long long off = 0;
+    P.Ls = c->nlev;
+    for (int l = c->nlev - 1; l >= 0; l--) {
+        const MGLevel &a = c->lev[l];
+        const long long nn = (long long)((a.nx + 3) | 1) * (a.ny + 3);
+        const long long need = 16 * nn + (nn + 15) / 16 * 16;
+        if ((long long)(a.nx + 1) * (a.ny + 1) > small_nodes || off + need > MG_SMEM) break;
+        P.L[l].su = (int)off; P.L[l].sb = (int)(off + 8 * nn); P.L[l].sm = (int)(off + 16 * nn);
+        off += need;
+        P.Ls = l;
+    }
+    // per level the tile that ends a pass soonest: its tiles go round the grid's CTAs, so a pass
+    // lasts (rounds) x (a tile's sweeps over its region, halo included, plus its fixed latencies,
+    // which cost about as much as 1500 nodes)
+    P.cap = MG_SMEM / 17 / 16 * 16;
+    const int workers = std::max(1, c->mg_grid - (P.Ls < c->nlev ? 1 : 0));
+    for (int l = 0; l < P.Ls; l++) {
+        double best = -1.0;
+        for (int tx = 8; tx <= 96; tx += 8)
+            for (int ty = 4; ty <= 96; ty += 4) {
+                const long long region = (long long)((tx + 2 * MG_HMAX) | 1) * (ty + 2 * MG_HMAX + 4);
+                if (region > P.cap) continue;
+                const long long nt = (long long)((c->lev[l].nx + tx) / tx) * ((c->lev[l].ny + ty) / ty);
+                const double rounds = (double)((nt + workers - 1) / workers);
+                const double cost = rounds * ((double)region + 1500.0);
+                if (best < 0.0 || cost < best) { best = cost; P.L[l].tx = tx; P.L[l].ty = ty; }
+            }
+    }
     P.omega = c->cfg.omega;
     P.eps = eps;
     P.alpha = fabs((double)(c->cfg.nx + 1) * (c->cfg.ny + 1) * P.L[0].ac) * 1.0;
@@ -406,25 +931,17 @@ static MGP mg_params(lepic_ctx *c, double eps, int mode) {
 
 int mg_init(lepic_ctx *c) {
     int occ = 0;
-    LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mg_solve, MG_THREADS, 0));
+    LCUDA(cudaFuncSetAttribute(k_mg_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM));
+    LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mg_solve, MGT, MG_SMEM));
     if (occ < 1) { c->last_err = "multigrid kernel does not fit on an SM"; return LEPIC_ECUDA; }
     c->mg_grid = c->num_sms * std::max(1, std::min(occ, (int)c->opt.ctas_per_sm));
     return LEPIC_OK;
 }
 
-static int launch_coop(lepic_ctx *c, void *fn, int grid, MGP &P) {
-    void *args[] = {&P};
-    LCUDA(cudaMemsetAsync(&c->dcnt->bar_arrived, 0, sizeof(unsigned long long) + sizeof(int), c->stream));
-    LCUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(MG_THREADS), args, 0, c->stream));
-    return LEPIC_OK;
-}
-
 int mg_solve(lepic_ctx *c, double eps, int mode) {
     MGP P = mg_params(c, eps, mode);
-    return launch_coop(c, (void *)k_mg_solve, c->mg_grid, P);
-}
-
-int mg_residual_stats(lepic_ctx *c) {
-    MGP P = mg_params(c, 0.0, 0);
-    return launch_coop(c, (void *)k_mg_stats, c->mg_grid, P);
+    void *args[] = {&P};
+    LCUDA(cudaMemsetAsync(&c->dcnt->bar_arrived, 0, sizeof(unsigned long long) + sizeof(int), c->stream));
+    LCUDA(cudaLaunchCooperativeKernel((void *)k_mg_solve, dim3(P.Ls == 0 ? 1 : c->mg_grid), dim3(MGT), args, MG_SMEM, c->stream));
+    return LEPIC_OK;
 }
