@@ -168,7 +168,7 @@ static int create_impl(lepic_ctx *c, const lepic_config *cfg, const int32_t *bcn
         B.cur = 0;
         LALLOC(B.acc, nn);
         LCUDA(cudaMemset(B.acc, 0, sizeof(unsigned long long) * nn));
-        B.max_items = c->ntiles + (int)(B.cap / 2048) + 16;
+        B.max_items = c->ntiles + (int)(B.cap / PUSH_CHUNK_MIN) + 16;
         LALLOC(B.items, B.max_items);
         B.prod_cap = (int)std::min<long long>(1 << 24, std::max<long long>(65536, B.cap / 50));
         LALLOC(B.prod, B.prod_cap);

@@ -11,9 +11,9 @@
 //            (plus a halo for particles that drifted since the sort); anything outside the
 //            window goes straight to the global uint64 grid.  Integer sums are associative,
 //            so the density is bit-reproducible whatever the atomic order.  A thread keeps a
-//            run of particles in one cell as its moments (count, sum fx, sum fy, sum fx fy)
-//            where those give the weights exactly, and adds each run once.
-// Work is dispensed dynamically: the sort's per-tile items first, then fixed-size chunks of
+//            run of particles in one cell as its moments (count, sum fx, sum fy, sum fx fy),
+//            which give the sum of the particles' weights exactly, and adds each run once.
+// Work is dispensed dynamically: the sort's per-tile items first, then chunks of
 // the unsorted tail (particles created by collisions since the sort); each CTA prefetches its
 // next iteration of the stream into L2 with bulk copies.
 //
@@ -22,7 +22,6 @@
 #include "lepic_internal.cuh"
 
 #define PUSH_THREADS 128
-#define PUSH_CHUNK 16384
 
 struct PushP {
     int nx, ny, S, W;
@@ -52,6 +51,8 @@ struct PushP {
     int tw, th, ntx, M, WX, WY, win;
     unsigned WX1, WY1;         // WX - 1, WY - 1
     int mom_up, mom_sup;       // LEPIC_DEP_SHIFT - 2S and LEPIC_DEP_SHIFT - S (moments deposit)
+    int rnd_sh;                // 2S - LEPIC_DEP_SHIFT, where that is positive (rounded weights)
+    uint32_t rnd_h, rnd_m;     // 2^(rnd_sh - 1) and 2^rnd_sh - 1
     long long xlim, ylim;      // nx<<S, ny<<S
     // the 3rd dimension (walls.cu): z per slot, its length, the end plates' potential and
     // phi for the electrons' test, the ions' loss factor hz 2 dt / zmax and the uB map
@@ -98,9 +99,6 @@ __device__ __forceinline__ void cic_weights_s(int S, uint32_t X, uint32_t Y, uin
         else if (sh < 0) w[k] <<= -sh;
     }
 }
-__device__ __forceinline__ void cic_weights(const PushP &P, uint32_t X, uint32_t Y, uint64_t *w) {
-    cic_weights_s(P.S, X, Y, w);
-}
 
 // one particle's weights added to the global accumulators of its cell's four nodes
 __device__ __forceinline__ void deposit_global(unsigned long long *acc, int S, int W, uint32_t X, uint32_t Y) {
@@ -113,35 +111,25 @@ __device__ __forceinline__ void deposit_global(unsigned long long *acc, int S, i
     atomicAdd(q + W, (unsigned long long)w[3]);
 }
 
-// the four accumulators of cell (ix, iy): the CTA's shared-memory window when the cell's four
-// nodes lie in it (window-relative cell 0 <= lx < WX - 1, 0 <= ly < WY - 1; an item without a
-// window has its origin far away), else the global grid
-__device__ __forceinline__ void add_cell(const PushP &P, unsigned long long *win, int ox, int oy,
-                                         int ix, int iy, const uint64_t *w) {
-    const int lx = ix - ox, ly = iy - oy;
-    unsigned long long *q;
-    int row;
-    if ((unsigned)lx < P.WX1 && (unsigned)ly < P.WY1) {
-        q = win + lx + ly * P.WX;
-        row = P.WX;
-    } else {
-        q = P.acc + ix + (long long)iy * P.W;
-        row = P.W;
-    }
-    atomicAdd(q, (unsigned long long)w[0]);
-    atomicAdd(q + 1, (unsigned long long)w[1]);
-    atomicAdd(q + row + 1, (unsigned long long)w[2]);
-    atomicAdd(q + row, (unsigned long long)w[3]);
-}
-
-// A run's moments added to cell (ix, iy) as node weights: n particles with offsets fx, fy
-// summed as sx = sum fx, sy = sum fy, sxy = sum fx fy give sum (A-fx)(A-fy), sum fx (A-fy),
-// sum fx fy, sum (A-fx) fy (A = 2^S).  Used when 2S <= LEPIC_DEP_SHIFT: every product is then
-// exact and only shifted up, so the run's weights equal the sum of its particles' cic_weights
-// bit for bit, for two 32-bit adds, one 32x32 product and one 64-bit add per particle.  The
-// shift up by 2^(LEPIC_DEP_SHIFT - 2S) is applied to the moments before the differences (a
-// shift distributes over sums modulo 2^64); n 2^(2S) shifted up is n 2^LEPIC_DEP_SHIFT.  Each
-// weight is formed just before its atomic, so that few 64-bit values are live at once.
+// A run's moments added to the four accumulators of cell (ix, iy) as node weights: the CTA's
+// shared-memory window when the cell's four nodes lie in it (window-relative cell 0 <= lx < WX - 1,
+// 0 <= ly < WY - 1; an item without a window has its origin far away), else the global grid.
+// n particles with offsets fx, fy summed as sx = sum fx, sy = sum fy, sxy = sum fx fy give
+// sum (A-fx)(A-fy), sum fx (A-fy), sum fx fy, sum (A-fx) fy (A = 2^S) exactly.
+//  * 2S <= LEPIC_DEP_SHIFT (grids above 512): the products are only shifted up, so the run's
+//    weights equal the sum of its particles' weights bit for bit, for two 32-bit adds, one 32x32
+//    product and one 64-bit add per particle.  The shift up by 2^(LEPIC_DEP_SHIFT - 2S) is
+//    applied to the moments before the differences (a shift distributes over sums modulo 2^64);
+//    n 2^(2S) shifted up is n 2^LEPIC_DEP_SHIFT.
+//  * RND (grids of 512 and below, sh = 2S - LEPIC_DEP_SHIFT of 2 or 4): each weight is rounded,
+//    (v + h) >> sh with h = 2^(sh-1), so a run's sum is (sum v + n h - sum of the bits cut off) >> sh.
+//    A being a multiple of 2^sh, the four products are fx fy, -fx fy, fx fy, -fx fy modulo 2^sh,
+//    so one remainder per particle, r = (fx fy + h) mod 2^sh, gives all four: the other sign's is
+//    2^sh - r, or 0 when r = 0.  n carries the run's count (bits 0..7), the number of nonzero r
+//    (8..15) and their sum (16..).  (Four rounded 64-bit weights per particle, accumulated one
+//    by one, took 0.986 ms per push of both species on 512^2 at 200 per cell, the moments 0.958.)
+// Each weight is formed just before its atomic, so that few 64-bit values are live at once.
+template <bool RND>
 __device__ __forceinline__ void add_run(const PushP &P, unsigned long long *win, int ox, int oy, int ix, int iy,
                                         uint32_t n, uint32_t sx, uint32_t sy, uint64_t sxy) {
     const int lx = ix - ox, ly = iy - oy;
@@ -153,6 +141,18 @@ __device__ __forceinline__ void add_run(const PushP &P, unsigned long long *win,
     } else {
         q = P.acc + ix + (long long)iy * P.W;
         row = P.W;
+    }
+    if (RND) {
+        const int sh = P.rnd_sh;
+        const int nh = (int)(n & 255u) << (sh - 1), cut = (int)(n >> 16), cut2 = ((int)((n >> 8) & 255u) << sh) - cut;
+        const uint64_t c2 = sxy + (uint64_t)(long long)(nh - cut);
+        atomicAdd(q + row + 1, (unsigned long long)(c2 >> sh));
+        const uint64_t d2 = sxy - (uint64_t)(long long)(nh - cut2);
+        const uint64_t ax = (uint64_t)sx << P.S, ay = (uint64_t)sy << P.S;
+        atomicAdd(q + 1, (unsigned long long)((ax - d2) >> sh));
+        atomicAdd(q + row, (unsigned long long)((ay - d2) >> sh));
+        atomicAdd(q, (unsigned long long)((((uint64_t)(n & 255u) << (2 * P.S)) - ax - ay + c2) >> sh));
+        return;
     }
     const uint64_t c2 = sxy << P.mom_up;
     atomicAdd(q + row + 1, (unsigned long long)c2);
@@ -389,8 +389,8 @@ __device__ __forceinline__ bool zstep(const PushP &P, int i, uint32_t &X, uint32
 // A work item's range is rounded down to multiples of 8 slots at both ends, so consecutive items
 // still tile the slot array exactly; particles a rounded range takes from a neighbouring
 // tile reach the global grid when they fall outside the window.
-template <int BMODE, bool GEN, bool MOVE, bool MOM, bool IND>
-__global__ void __launch_bounds__(PUSH_THREADS, 8) k_push_deposit(PushP P) {
+template <int BMODE, bool GEN, bool MOVE, bool RND, bool IND>
+__global__ void __launch_bounds__(PUSH_THREADS, PUSH_CTAS_PER_SM) k_push_deposit(PushP P) {
     extern __shared__ unsigned long long win[];
     __shared__ int s_tile, s_start, s_end;
     __shared__ unsigned int s_lost;
@@ -399,6 +399,7 @@ __global__ void __launch_bounds__(PUSH_THREADS, 8) k_push_deposit(PushP P) {
     const long long ind_old = IND ? cnt->ind_old[P.sp] : 0;
     const int n_items = cnt->n_items[P.sp];
     const long long tail0 = n_sorted & ~7ll;
+    const int tail_chunk = push_chunk(n_slots - tail0, gridDim.x);
     for (;;) {
         if (threadIdx.x == 0) {
             unsigned int w = atomicAdd(&cnt->work_next[P.sp], 1u);
@@ -406,9 +407,9 @@ __global__ void __launch_bounds__(PUSH_THREADS, 8) k_push_deposit(PushP P) {
                 WorkItem it = P.items[w];
                 s_tile = it.tile; s_start = it.start & ~7; s_end = it.end & ~7;
             } else {
-                long long st = tail0 + (long long)(w - n_items) * PUSH_CHUNK;
+                long long st = tail0 + (long long)(w - n_items) * tail_chunk;
                 if (st >= n_slots) { s_tile = -2; s_start = s_end = 0; }
-                else { s_tile = -1; s_start = (int)st; s_end = (int)min(st + PUSH_CHUNK, n_slots); }
+                else { s_tile = -1; s_start = (int)st; s_end = (int)min(st + tail_chunk, n_slots); }
             }
             s_lost = 0;
         }
@@ -490,8 +491,9 @@ __global__ void __launch_bounds__(PUSH_THREADS, 8) k_push_deposit(PushP P) {
                 vy[0] = b0.x; vy[1] = b0.y; vy[2] = b0.z; vy[3] = b0.w;
                 vz[0] = c0.x; vz[1] = c0.y; vz[2] = c0.z; vz[3] = c0.w;
             }
-            int rkey = -1, rix = 0, riy = 0;   // the current run of equal cells
-            uint64_t rw[4] = {0, 0, 0, 0};     // its weights, or (MOM) its moments n, sx, sy, sxy
+            int rkey = -1, rix = 0, riy = 0;         // the current run of equal cells
+            uint32_t rn = 0, rsx = 0, rsy = 0;       // its moments n, sum fx, sum fy, sum fx fy
+            uint64_t rxy = 0;
             const uint32_t fmask = (1u << P.S) - 1u;
             if (grp_ok) {
 #pragma unroll
@@ -510,27 +512,19 @@ __global__ void __launch_bounds__(PUSH_THREADS, 8) k_push_deposit(PushP P) {
                     }
                     if (!alive) continue;
                     const int key = ix + iy * P.W;
-                    if (MOM) {
-                        const uint32_t fx = X[p] & fmask, fy = Y[p] & fmask;
-                        const uint64_t fxy = (uint64_t)fx * fy;
-                        if (key != rkey) {
-                            if (rkey >= 0)
-                                add_run(P, win, ox, oy, rix, riy, (uint32_t)rw[0], (uint32_t)rw[1], (uint32_t)rw[2], rw[3]);
-                            rkey = key; rix = ix; riy = iy;
-                            rw[0] = 1; rw[1] = fx; rw[2] = fy; rw[3] = fxy;
-                        } else {
-                            rw[0] += 1; rw[1] += fx; rw[2] += fy; rw[3] += fxy;
-                        }
-                        continue;
+                    const uint32_t fx = X[p] & fmask, fy = Y[p] & fmask;
+                    const uint64_t fxy = (uint64_t)fx * fy;
+                    uint32_t one = 1u;
+                    if (RND) {
+                        const uint32_t r = ((uint32_t)fxy + P.rnd_h) & P.rnd_m;
+                        one = (r << 16) + (r ? 257u : 1u);
                     }
-                    uint64_t w[4];
-                    cic_weights(P, X[p], Y[p], w);
                     if (key != rkey) {
-                        if (rkey >= 0) add_cell(P, win, ox, oy, rix, riy, rw);
+                        if (rkey >= 0) add_run<RND>(P, win, ox, oy, rix, riy, rn, rsx, rsy, rxy);
                         rkey = key; rix = ix; riy = iy;
-                        rw[0] = w[0]; rw[1] = w[1]; rw[2] = w[2]; rw[3] = w[3];
+                        rn = one; rsx = fx; rsy = fy; rxy = fxy;
                     } else {
-                        rw[0] += w[0]; rw[1] += w[1]; rw[2] += w[2]; rw[3] += w[3];
+                        rn += one; rsx += fx; rsy += fy; rxy += fxy;
                     }
                 }
                 if (MOVE) {
@@ -545,13 +539,7 @@ __global__ void __launch_bounds__(PUSH_THREADS, 8) k_push_deposit(PushP P) {
             // after the sort) meet at the same shared-memory words, and the serialised atomics
             // cost less issue than any warp-level combination of the runs (a group-masked warp
             // reduction measured 16 % slower on the whole push, a segmented shuffle scan 4 %)
-            if (rkey >= 0) {
-                if (MOM) {
-                    add_run(P, win, ox, oy, rix, riy, (uint32_t)rw[0], (uint32_t)rw[1], (uint32_t)rw[2], rw[3]);
-                } else {
-                    add_cell(P, win, ox, oy, rix, riy, rw);
-                }
-            }
+            if (rkey >= 0) add_run<RND>(P, win, ox, oy, rix, riy, rn, rsx, rsy, rxy);
         }
         // lost-particle count: one atomic per warp, then per CTA
         for (int o = 16; o > 0; o >>= 1) lost += __shfl_xor_sync(0xffffffffu, lost, o);
@@ -575,35 +563,35 @@ __global__ void __launch_bounds__(PUSH_THREADS, 8) k_push_deposit(PushP P) {
 }
 
 // the kernel's dynamic shared-memory limit, set once per device (this also loads the kernel)
-template <int BMODE, bool GEN, bool MOVE, bool MOM, bool IND>
+template <int BMODE, bool GEN, bool MOVE, bool RND, bool IND>
 static int set_push_attr(lepic_ctx *c) {
     static bool attr_set[64] = {false};
     if (!attr_set[c->dev & 63]) {
-        LCUDA(cudaFuncSetAttribute(k_push_deposit<BMODE, GEN, MOVE, MOM, IND>,
+        LCUDA(cudaFuncSetAttribute(k_push_deposit<BMODE, GEN, MOVE, RND, IND>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
         attr_set[c->dev & 63] = true;
     }
     return LEPIC_OK;
 }
 
-template <int BMODE, bool GEN, bool MOVE, bool MOM, bool IND>
+template <int BMODE, bool GEN, bool MOVE, bool RND, bool IND>
 static int launch_one(lepic_ctx *c, PushP &P, size_t smem) {
-    const int ra = set_push_attr<BMODE, GEN, MOVE, MOM, IND>(c);
+    const int ra = set_push_attr<BMODE, GEN, MOVE, RND, IND>(c);
     if (ra != LEPIC_OK) return ra;
     int occ = 0;
-    LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_push_deposit<BMODE, GEN, MOVE, MOM, IND>,
+    LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_push_deposit<BMODE, GEN, MOVE, RND, IND>,
                                                         PUSH_THREADS, smem));
-    k_push_deposit<BMODE, GEN, MOVE, MOM, IND><<<c->num_sms * std::max(1, occ), PUSH_THREADS, smem, c->stream>>>(P);
+    k_push_deposit<BMODE, GEN, MOVE, RND, IND><<<c->num_sms * std::max(1, occ), PUSH_THREADS, smem, c->stream>>>(P);
     LCUDA(cudaGetLastError());
     return LEPIC_OK;
 }
 
 // ind: the fast mover reading through a pending permutation (only without the general mover)
-template <int BMODE, bool MOM>
+template <int BMODE, bool RND>
 static int launch_m(lepic_ctx *c, PushP &P, size_t smem, bool gen, bool move, bool ind) {
-    if (!move) return launch_one<BMODE, false, false, MOM, false>(c, P, smem);
-    if (gen) return launch_one<BMODE, true, true, MOM, false>(c, P, smem);
-    return ind ? launch_one<BMODE, false, true, MOM, true>(c, P, smem) : launch_one<BMODE, false, true, MOM, false>(c, P, smem);
+    if (!move) return launch_one<BMODE, false, false, RND, false>(c, P, smem);
+    if (gen) return launch_one<BMODE, true, true, RND, false>(c, P, smem);
+    return ind ? launch_one<BMODE, false, true, RND, true>(c, P, smem) : launch_one<BMODE, false, true, RND, false>(c, P, smem);
 }
 
 // The mover that reads through a pending permutation, configured (and so loaded) ahead of its
@@ -611,8 +599,8 @@ static int launch_m(lepic_ctx *c, PushP &P, size_t smem, bool gen, bool move, bo
 // so that the first push after a deferred sort pays no kernel loading.
 template <int BMODE>
 static int preload_ind_b(lepic_ctx *c) {
-    return 2 * c->S <= LEPIC_DEP_SHIFT ? set_push_attr<BMODE, false, true, true, true>(c)
-                                       : set_push_attr<BMODE, false, true, false, true>(c);
+    return 2 * c->S > LEPIC_DEP_SHIFT ? set_push_attr<BMODE, false, true, true, true>(c)
+                                      : set_push_attr<BMODE, false, true, false, true>(c);
 }
 int push_preload_ind(lepic_ctx *c, int s) {
     const lepic_config &g = c->cfg;
@@ -623,11 +611,12 @@ int push_preload_ind(lepic_ctx *c, int s) {
     return preload_ind_b<0>(c);
 }
 
-// moments deposit where the weights are exact (2S <= LEPIC_DEP_SHIFT, grids of 1024 and up)
+// rounded weights where the products have more bits than the accumulators (2S > LEPIC_DEP_SHIFT,
+// grids of 512 and below)
 template <int BMODE>
 static int launch_b(lepic_ctx *c, PushP &P, size_t smem, bool gen, bool move, bool ind) {
-    return 2 * P.S <= LEPIC_DEP_SHIFT ? launch_m<BMODE, true>(c, P, smem, gen, move, ind)
-                                      : launch_m<BMODE, false>(c, P, smem, gen, move, ind);
+    return 2 * P.S > LEPIC_DEP_SHIFT ? launch_m<BMODE, true>(c, P, smem, gen, move, ind)
+                                     : launch_m<BMODE, false>(c, P, smem, gen, move, ind);
 }
 
 // Refluxing (part_expmover.f90:445-470), one thread per event of this species' push: vx from
@@ -812,6 +801,9 @@ int push_deposit(lepic_ctx *c, int it, bool move) {
         P.inv2S = 1.0f / (float)(1u << c->S);
         P.mom_up = LEPIC_DEP_SHIFT - 2 * c->S;
         P.mom_sup = LEPIC_DEP_SHIFT - c->S;
+        P.rnd_sh = std::max(0, 2 * c->S - LEPIC_DEP_SHIFT);
+        P.rnd_m = (1u << P.rnd_sh) - 1u;
+        P.rnd_h = (P.rnd_m + 1u) >> 1;
         P.pbc = g.flag_pbc; P.spec = g.flag_spec; P.nmn = g.flag_nmn;
         P.negion_nmn = (g.charge[s] < 0 && g.mass[s] >= amu && g.flag_nmn == 1) ? 1 : 0;
         P.step_key = (uint32_t)(g.seed * 0x2545F491ull) ^ ((uint32_t)it * 0x27D4EB2Fu) ^ ((uint32_t)s * 0x165667B1u);

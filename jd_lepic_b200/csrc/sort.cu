@@ -10,7 +10,7 @@
 //   4. per-key segment sort of the slot indices (bitonic, ascending; segments already in
 //      order are skipped) -> stable again
 //   5. gather of the 5 SoA fields into the other buffer, holes dropped
-//   6. push work list: per tile, chunks of CHUNK particles
+//   6. push work list: per tile, chunks of push_chunk() particles
 // so the result is bit-identical to the reference's, independent of thread timing.
 // The key is the reference's cell index when tile_w = nx, tile_h = 1; other tile shapes
 // order cells tile by tile (the push kernel then stages a compact node window per tile).
@@ -22,7 +22,6 @@
 #include "lepic_internal.cuh"
 
 #define SORT_THREADS 256
-#define PUSH_CHUNK 16384
 #define SEG_WARP_MAX 256
 #define SEG_BLOCK_MAX 8192
 #define SEG_CHECK_STEPS 4
@@ -356,11 +355,12 @@ __global__ void k_gather(const int *perm, const int *offsets, long long nkeys, c
     }
 }
 
-// per tile: ceil(count / CHUNK) work items; single block, fixed order
+// per tile: ceil(count / chunk) work items; single block, fixed order
 __global__ void k_items(const int *offsets, int ntiles, int keys_per_tile, WorkItem *items,
-                        int max_items, DevCounters *cnt, int sp, long long nkeys) {
+                        int max_items, DevCounters *cnt, int sp, long long nkeys, int ctas) {
     __shared__ int s[1024];
     __shared__ int carry;
+    const int chunk = push_chunk(offsets[nkeys], ctas);
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     for (int base = 0; base < ntiles; base += 1024) {
@@ -369,7 +369,7 @@ __global__ void k_items(const int *offsets, int ntiles, int keys_per_tile, WorkI
         if (t < ntiles) {
             st = offsets[(long long)t * keys_per_tile];
             en = offsets[(long long)(t + 1) * keys_per_tile];
-            ni = (en - st + PUSH_CHUNK - 1) / PUSH_CHUNK;
+            ni = (en - st + chunk - 1) / chunk;
         }
         s[threadIdx.x] = ni;
         __syncthreads();
@@ -385,8 +385,8 @@ __global__ void k_items(const int *offsets, int ntiles, int keys_per_tile, WorkI
             if (idx < max_items) {
                 WorkItem w;
                 w.tile = t;
-                w.start = st + q * PUSH_CHUNK;
-                w.end = min(en, st + (q + 1) * PUSH_CHUNK);
+                w.start = st + q * chunk;
+                w.end = min(en, st + (q + 1) * chunk);
                 w.pad = 0;
                 items[idx] = w;
             }
@@ -453,7 +453,7 @@ int sort_species(lepic_ctx *c, int sp, bool defer) {
                                                        B.VY[cur], B.VZ[cur], B.X[nxt], B.Y[nxt], B.VX[nxt],
                                                        B.VY[nxt], B.VZ[nxt], B.Z[cur], B.Z[nxt]);
     k_items<<<1, 1024, 0, c->stream>>>(c->offsets, c->ntiles, c->tw * c->th, B.items, B.max_items,
-                                       c->dcnt, sp, nk);
+                                       c->dcnt, sp, nk, c->num_sms * PUSH_CTAS_PER_SM);
     LCUDA(cudaGetLastError());
     // the cell lists of this order (sorting.f90's Plist) for the DSMC target search
     if (B.cell_off)
