@@ -235,20 +235,85 @@ __device__ __forceinline__ void warp_sort64(int &v0, int &v1, int lane) {
     }
 }
 
+// A long segment put in order by one warp.  The slots that one work unit scatters into a segment
+// arrive in ascending order, and the units' slot ranges are disjoint: with the unit of the
+// segment's middle slot as the main one (nearly all of the cell's particles stay in its tile's
+// item), the ordered segment is the slots below the main range, then the main ones as they
+// are, then those above it.  So the main slots are compacted (into tmp and back) and only the
+// others, at most SEG_WARP_MAX, are sorted.  Returns false, with
+// the segment untouched, when there are more or the main slots are not ascending.
+// (A bitonic sort of the whole segment by a 512-thread CTA took 2.6 ms per species on 512^2 cells
+// with a Gaussian peak of 1000 per cell; a whole step there
+// 3.00 -> 2.46 ms with seg_merge.)
+__device__ __forceinline__ bool seg_merge(int *perm, int *tmp, int t0, int n, const WorkItem *items, int ni, long long ns,
+                                          long long n_slots, int *buf, int lane) {
+    const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+    const int e = perm[t0 + (n >> 1)];
+    long long ms, me;                    // the main unit's slots
+    if (e < ns) {
+        int lo = 0, hi = ni;             // the last item that starts at or before e
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (items[mid].start <= e) lo = mid;
+            else hi = mid;
+        }
+        ms = items[lo].start;
+        me = items[lo].end;
+    } else {
+        ms = ns + (e - ns) / SCATTER_CHUNK * SCATTER_CHUNK;
+        me = min(ms + SCATTER_CHUNK, n_slots);
+    }
+    int m = 0, d = 0, dl = 0, carry = -1;
+    bool bad = false;
+    for (int q0 = 0; q0 < n; q0 += 128) {
+        int v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = q0 + 32 * u + lane < n ? perm[t0 + q0 + 32 * u + lane] : -1;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const bool in = q0 + 32 * u + lane < n, low = in && v[u] < ms, high = in && v[u] >= me, main = in && !low && !high;
+            const unsigned mm = __ballot_sync(full, main), mo = __ballot_sync(full, low || high);
+            const int prev_lane = 31 - __clz(mm & below);
+            const int pv = __shfl_sync(full, v[u], prev_lane & 31);
+            if (main) {
+                bad = bad || (prev_lane >= 0 ? pv : carry) > v[u];
+                tmp[t0 + m + __popc(mm & below)] = v[u];
+            }
+            const int k = d + __popc(mo & below);
+            if ((low || high) && k < SEG_WARP_MAX) buf[k] = v[u];
+            const int last = __shfl_sync(full, v[u], (31 - __clz(mm)) & 31);
+            if (mm) carry = last;
+            m += __popc(mm);
+            d += __popc(mo);
+            dl += __popc(__ballot_sync(full, low));
+        }
+    }
+    if (__any_sync(full, bad) || d > SEG_WARP_MAX) return false;
+    __syncwarp();
+    bitonic_sort(buf, d, lane, 32, WarpSync());
+    for (int q = lane; q < d; q += 32) perm[t0 + (q < dl ? q : m + q)] = buf[q];
+#pragma unroll 4
+    for (int q = lane; q < m; q += 32) perm[t0 + dl + q] = tmp[t0 + q];
+    __syncwarp();
+    return true;
+}
+
 // A warp takes 32 consecutive segments: one coalesced load of their bounds, then one pass over
 // their slot lists in 32-wide steps that marks each segment holding a descending adjacent pair
 // (the segment of a position is found by a binary search over the 32 bounds held in the lanes);
-// only the marked segments are sorted: up to 64 slots in registers, up to SEG_WARP_MAX in the
-// warp's shared memory, longer ones listed for k_segsort_big.  (One segment per warp, each with
+// only the marked segments are put in order: up to 64 slots in registers, longer ones by
+// seg_merge, those it cannot take listed for k_segsort_big.  (One segment per warp, each with
 // its own dependent loads of bounds and slots, was latency-bound on the segments in order.)
-__global__ void k_segsort_warp(const int *offsets, long long nkeys, int *perm, int *bigseg,
-                               DevCounters *cnt) {
+__global__ void k_segsort_warp(const int *offsets, long long nkeys, int *perm, int *tmp, int *bigseg,
+                               const WorkItem *items, DevCounters *cnt, int sp) {
     __shared__ int buf[SORT_THREADS / 32][SEG_WARP_MAX];
     const unsigned full = 0xffffffffu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
     const long long ngroups = (nkeys + 31) / 32;
+    const long long n_slots = cnt->n_slots[sp], n_sorted = min(cnt->n_sorted[sp], n_slots);
+    const int ni = cnt->n_items[sp];
     for (long long gi = gw; gi < ngroups; gi += nw) {
         const long long k = gi * 32 + lane;
         const int s0 = offsets[k < nkeys ? k : nkeys];
@@ -288,14 +353,7 @@ __global__ void k_segsort_warp(const int *offsets, long long nkeys, int *perm, i
                 warp_sort64(v0, v1, lane);
                 if (lane < n) perm[t0 + lane] = v0;
                 if (lane + 32 < n) perm[t0 + lane + 32] = v1;
-            } else if (n <= SEG_WARP_MAX) {
-                int *a = buf[warp];
-                for (int q = lane; q < n; q += 32) a[q] = perm[t0 + q];
-                __syncwarp();
-                bitonic_sort(a, n, lane, 32, WarpSync());
-                for (int q = lane; q < n; q += 32) perm[t0 + q] = a[q];
-                __syncwarp();
-            } else if (lane == 0) {
+            } else if (!seg_merge(perm, tmp, t0, n, items, ni, n_sorted, n_slots, buf[warp], lane) && lane == 0) {
                 const int slot = atomicAdd(&cnt->n_big, 1);
                 bigseg[slot] = (int)(gi * 32 + l);
             }
@@ -446,7 +504,7 @@ int sort_species(lepic_ctx *c, int sp, bool defer) {
     k_scan_final<<<nb, SORT_THREADS, 0, c->stream>>>(c->counts, nk, c->blocksums, c->offsets);
     LCUDA(cudaMemcpyAsync(c->cursor, c->offsets, sizeof(int) * nk, cudaMemcpyDeviceToDevice, c->stream));
     k_scatter<<<grid, SORT_THREADS, 0, c->stream>>>(c->keys, B.items, c->dcnt, sp, c->cursor, perm);
-    k_segsort_warp<<<grid, SORT_THREADS, 0, c->stream>>>(c->offsets, nk, perm, c->bigseg, c->dcnt);
+    k_segsort_warp<<<grid, SORT_THREADS, 0, c->stream>>>(c->offsets, nk, perm, c->keys, c->bigseg, B.items, c->dcnt, sp);
     k_segsort_big<<<c->num_sms, 512, 0, c->stream>>>(c->offsets, perm, c->bigseg, c->dcnt);
     if (!defer)
         k_gather<<<grid, SORT_THREADS, 0, c->stream>>>(perm, c->offsets, nk, B.X[cur], B.Y[cur], B.VX[cur],
