@@ -94,21 +94,26 @@ __global__ void k_efield_interior(int nx, int ny, double h1, double h2, const do
         }
     }
 }
-// Pass 2, periodic rows (:68-82) when part == 0, then the Neumann column (:52-63) when
-// part == 1; one thread per column / row.  The reference visits row 1 first, so its periodic
-// copies read column 1 before the Neumann step zeroes Ex there: two launches keep that order.
+// Pass 2, periodic rows (:68-82) when part == 0, one thread per column, then the Neumann column
+// (:52-63) when part == 1, one warp per row (a thread that looked along its whole row for a Neumann
+// node took 43 us on 384 x 256 cells, its loads one after another; the warp 3 us).  The
+// reference visits row 1 first, so its periodic copies read column 1 before the Neumann step
+// zeroes Ex there: two launches keep that order.
 __global__ void k_efield_nmn_pbc(int nx, int ny, double h2, const double *phi, const int8_t *bc,
                                  double2 *E, int part) {
     const int W = nx + 3;
     int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (part == 1 && t >= 1 && t <= ny + 1) { // Neumann: any node of row iy with bcnd == -2
-        int iy = t;
-        for (int ix = 1; ix <= nx + 1; ix++) {
-            if (bc[ix + iy * W] != -2) continue;
+    if (part == 1) { // Neumann: any node of row iy with bcnd == -2
+        const int iy = (t >> 5) + 1, lane = t & 31;
+        if (iy > ny + 1) return;
+        bool any = false;
+        for (int ix = 1 + lane; ix <= nx + 1; ix += 32) any = any || bc[ix + iy * W] == -2;
+        if (__any_sync(0xffffffffu, any) && lane == 0) {
             E[1 + iy * W].x = 0.0;
             if (iy > 1 && iy < ny + 1)
                 E[1 + iy * W].y = -(phi[1 + (iy + 1) * W] - phi[1 + (iy - 1) * W]) / (2.0 * h2);
         }
+        return;
     }
     if (part == 0 && t >= 1 && t <= nx + 1) { // periodic: node (ix, 1)
         int ix = t;
@@ -219,8 +224,8 @@ int field_calc_efield(lepic_ctx *c) {
     k_efield_interior<<<grid, 256, 0, c->stream>>>(nx, ny, c->cfg.dx, c->cfg.dy, c->phi, c->bc8, E1, E0);
     if (c->cfg.flag_pbc || c->cfg.flag_nmn) // the passes test the labels, as Efield.f90:43-82 does
         for (int part = 0; part < 2; part++)
-            k_efield_nmn_pbc<<<div_up(std::max(nx, ny) + 2, 256), 256, 0, c->stream>>>(nx, ny, c->cfg.dy,
-                                                                                       c->phi, c->bc8, E0, part);
+            k_efield_nmn_pbc<<<div_up(part ? 32ll * (ny + 1) : nx + 2, 256), 256, 0, c->stream>>>(nx, ny, c->cfg.dy, c->phi,
+                                                                                                  c->bc8, E0, part);
     int grid2 = (int)std::min<long long>(div_up(c->nn, 256), (long long)c->num_sms * 16);
     k_efield_walls<<<grid2, 256, 0, c->stream>>>(nx, ny, c->bc8, E0, E1, c->Ef);
     LCUDA(cudaGetLastError());
