@@ -63,6 +63,7 @@ static void free_all(lepic_ctx *c) {
     if (c->ev_down) cudaEventDestroy(c->ev_down);
     if (c->ev_up) cudaEventDestroy(c->ev_up);
     F(c->snap);
+    io_free(c);
     if (c->stream) cudaStreamDestroy(c->stream);
 }
 
@@ -414,77 +415,7 @@ extern "C" int lepic_gpu_sync(lepic_ctx *c) {
 }
 
 // ---------------------------------------------------------------------------------------
-// particles
-int particles_put(lepic_ctx *c, int sp, const double *vxp, long long n) {
-    SpeciesBuf &B = c->sp[sp];
-    if (n < 0 || n > B.cap) { c->last_err = "particle count exceeds capacity"; return LEPIC_ECAPACITY; }
-    const lepic_config &g = c->cfg;
-    const double sx = (double)(1u << c->S) / g.dx, sy = (double)(1u << c->S) / g.dy;
-    const long long xl = (long long)g.nx << c->S, yl = (long long)g.ny << c->S;
-    std::vector<uint32_t> X(n), Y(n);
-    std::vector<float> VX(n), VY(n), VZ(n), Z(B.Z[0] ? n : 0);
-    for (long long k = 0; k < n; k++) {
-        const double *p = vxp + 6 * k;
-        long long xi = llround(p[0] * sx), yi = llround(p[1] * sy);
-        if (xi < 0 || xi >= xl || yi < 0 || yi >= yl) { c->last_err = "particle outside the box"; return LEPIC_EINVAL; }
-        X[k] = (uint32_t)xi; Y[k] = (uint32_t)yi;
-        VX[k] = (float)p[3]; VY[k] = (float)p[4]; VZ[k] = (float)p[5];
-        if (B.Z[0]) Z[k] = (float)p[2];
-    }
-    const int cur = B.cur;
-    if (n > 0 && B.Z[0]) LCUDA(cudaMemcpyAsync(B.Z[cur], Z.data(), 4 * n, cudaMemcpyHostToDevice, c->stream));
-    if (n > 0) {
-        LCUDA(cudaMemcpyAsync(B.X[cur], X.data(), 4 * n, cudaMemcpyHostToDevice, c->stream));
-        LCUDA(cudaMemcpyAsync(B.Y[cur], Y.data(), 4 * n, cudaMemcpyHostToDevice, c->stream));
-        LCUDA(cudaMemcpyAsync(B.VX[cur], VX.data(), 4 * n, cudaMemcpyHostToDevice, c->stream));
-        LCUDA(cudaMemcpyAsync(B.VY[cur], VY.data(), 4 * n, cudaMemcpyHostToDevice, c->stream));
-        LCUDA(cudaMemcpyAsync(B.VZ[cur], VZ.data(), 4 * n, cudaMemcpyHostToDevice, c->stream));
-    }
-    LCUDA(cudaStreamSynchronize(c->stream));
-    long long v = n;
-    int zero = 0;
-    LCUDA(cudaMemcpy(&c->dcnt->n_slots[sp], &v, sizeof(v), cudaMemcpyHostToDevice));
-    LCUDA(cudaMemcpy(&c->dcnt->n_alive[sp], &v, sizeof(v), cudaMemcpyHostToDevice));
-    v = 0;
-    LCUDA(cudaMemcpy(&c->dcnt->n_sorted[sp], &v, sizeof(v), cudaMemcpyHostToDevice));
-    LCUDA(cudaMemcpy(&c->dcnt->n_items[sp], &zero, sizeof(int), cudaMemcpyHostToDevice));
-    B.ordered = false;
-    return LEPIC_OK;
-}
-
-int particles_get(lepic_ctx *c, int sp, double *vxp, long long cap, long long *n_out) {
-    int r = sync_counters(c);
-    if (r != LEPIC_OK) return r;
-    SpeciesBuf &B = c->sp[sp];
-    const long long ns = c->hcnt->n_slots[sp];
-    std::vector<uint32_t> X(ns), Y(ns);
-    std::vector<float> VX(ns), VY(ns), VZ(ns), Z(B.Z[0] ? ns : 0);
-    const int cur = B.cur;
-    if (ns > 0 && B.Z[0]) LCUDA(cudaMemcpy(Z.data(), B.Z[cur], 4 * ns, cudaMemcpyDeviceToHost));
-    if (ns > 0) {
-        LCUDA(cudaMemcpy(X.data(), B.X[cur], 4 * ns, cudaMemcpyDeviceToHost));
-        LCUDA(cudaMemcpy(Y.data(), B.Y[cur], 4 * ns, cudaMemcpyDeviceToHost));
-        LCUDA(cudaMemcpy(VX.data(), B.VX[cur], 4 * ns, cudaMemcpyDeviceToHost));
-        LCUDA(cudaMemcpy(VY.data(), B.VY[cur], 4 * ns, cudaMemcpyDeviceToHost));
-        LCUDA(cudaMemcpy(VZ.data(), B.VZ[cur], 4 * ns, cudaMemcpyDeviceToHost));
-    }
-    const lepic_config &g = c->cfg;
-    const double ux = g.dx * std::ldexp(1.0, -c->S), uy = g.dy * std::ldexp(1.0, -c->S);
-    long long k = 0;
-    for (long long i = 0; i < ns; i++) {
-        if (std::isnan(VX[i])) continue;
-        if (vxp && k < cap) {
-            double *p = vxp + 6 * k;
-            p[0] = (double)X[i] * ux; p[1] = (double)Y[i] * uy; p[2] = B.Z[0] ? (double)Z[i] : 0.0;
-            p[3] = VX[i]; p[4] = VY[i]; p[5] = VZ[i];
-        }
-        k++;
-    }
-    if (n_out) *n_out = k;
-    if (vxp && k > cap) { c->last_err = "output capacity too small"; return LEPIC_ECAPACITY; }
-    return LEPIC_OK;
-}
-
+// particles (particles_put and particles_get are in backup.cu)
 struct LoadP {
     int nx, ny, S, ntype, profile;
     long long n;

@@ -21,6 +21,8 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
+#include <thread>
 #include <vector>
 #include "lepic_internal.cuh"
 
@@ -91,6 +93,211 @@ __global__ void k_unpack(const double *in, long long n, long long dst, double sx
         VX[s] = (float)p[3]; VY[s] = (float)p[4]; VZ[s] = (float)p[5];
         if (Z) Z[s] = (float)p[2];
     }
+}
+
+// ---------------------------------------------------------------------------------------
+// Particles to and from the host's FP64 vxp(6, n): the records cross in chunks of IO_CHUNK through
+// two pinned buffers, the conversion to and from the device's arrays is done on the device, and
+// each chunk's host copy (by a few threads: one thread's copy, and its page faults on a new array,
+// are slower than the bus) runs beside the transfer and conversion of the other.  Bound by those
+// host copies: 48 B per particle each way.  (Converted by one host thread between plain copies,
+// put + sort + deposit + get of 2 x 1.3 M particles took 67 ms; so 22 ms, most of it
+// the page faults of the fresh host arrays.)
+#define IO_CHUNK (1ll << 17)          // particles per chunk (a multiple of BK_BLOCK): 6.3 MB
+struct IoStage {
+    long long cap = 0;                // particles per buffer
+    double *d[2] = {nullptr, nullptr}, *h[2] = {nullptr, nullptr};
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    long long blocks = 0;             // entries of the two below
+    int *counts = nullptr;
+    long long *off = nullptr;
+    int *bad = nullptr;               // a particle outside the box (device), and its pinned mirror
+    int *hbad = nullptr;
+};
+
+void io_free(lepic_ctx *c) {
+    IoStage *S = (IoStage *)c->io;
+    if (!S) return;
+    for (int k = 0; k < 2; k++) {
+        if (S->d[k]) cudaFree(S->d[k]);
+        if (S->h[k]) cudaFreeHost(S->h[k]);
+        if (S->ev[k]) cudaEventDestroy(S->ev[k]);
+    }
+    if (S->counts) cudaFree(S->counts);
+    if (S->off) cudaFree(S->off);
+    if (S->bad) cudaFree(S->bad);
+    if (S->hbad) cudaFreeHost(S->hbad);
+    delete S;
+    c->io = nullptr;
+}
+
+// the context's staging for n particles (at most IO_CHUNK at a time) and nb counting blocks; kept
+// until the context is destroyed
+static int io_stage(lepic_ctx *c, long long n, long long nb, IoStage **out) {
+    if (!c->io) c->io = new (std::nothrow) IoStage;
+    IoStage *S = (IoStage *)c->io;
+    if (!S) { c->last_err = "particle staging: out of host memory"; return LEPIC_ENOMEM; }
+    auto fail = [&](cudaError_t e) {
+        c->last_err = std::string("particle staging: ") + cudaGetErrorString(e);
+        io_free(c);
+        return LEPIC_ENOMEM;
+    };
+    cudaError_t e;
+    if (!S->bad) {
+        if ((e = cudaMalloc((void **)&S->bad, sizeof(int))) != cudaSuccess) return fail(e);
+        if ((e = cudaMallocHost((void **)&S->hbad, sizeof(int))) != cudaSuccess) return fail(e);
+        for (int k = 0; k < 2; k++)
+            if ((e = cudaEventCreateWithFlags(&S->ev[k], cudaEventDisableTiming)) != cudaSuccess) return fail(e);
+    }
+    const long long want = std::min(IO_CHUNK, (n + BK_BLOCK - 1) / BK_BLOCK * BK_BLOCK);
+    if (S->cap < want) {
+        S->cap = 0;
+        for (int k = 0; k < 2; k++) {
+            if (S->d[k]) cudaFree(S->d[k]);
+            if (S->h[k]) cudaFreeHost(S->h[k]);
+            S->d[k] = S->h[k] = nullptr;
+            if ((e = cudaMalloc((void **)&S->d[k], 48 * want)) != cudaSuccess) return fail(e);
+            if ((e = cudaMallocHost((void **)&S->h[k], 48 * want)) != cudaSuccess) return fail(e);
+        }
+        S->cap = want;
+    }
+    if (S->blocks < nb) {
+        if (S->counts) cudaFree(S->counts);
+        if (S->off) cudaFree(S->off);
+        S->counts = nullptr; S->off = nullptr; S->blocks = 0;
+        if ((e = cudaMalloc((void **)&S->counts, sizeof(int) * nb)) != cudaSuccess) return fail(e);
+        if ((e = cudaMalloc((void **)&S->off, sizeof(long long) * (nb + 1))) != cudaSuccess) return fail(e);
+        S->blocks = nb;
+    }
+    *out = S;
+    return LEPIC_OK;
+}
+
+// memcpy by up to four threads
+static void host_copy(void *dst, const void *src, size_t bytes) {
+    const size_t kPart = 1 << 20;
+    const int nt = (int)std::min<size_t>(std::min(4u, std::max(1u, std::thread::hardware_concurrency())), bytes / kPart);
+    if (nt < 2) { std::memcpy(dst, src, bytes); return; }
+    const size_t part = (bytes / nt + 4095) / 4096 * 4096;
+    std::vector<std::thread> pool;
+    size_t o = part;
+    try {
+        for (int t = 1; t < nt && o < bytes; t++) {
+            const size_t k = std::min(part, bytes - o);
+            pool.emplace_back([=] { std::memcpy((char *)dst + o, (const char *)src + o, k); });
+            o += k;
+        }
+    } catch (...) { }                 // no more threads: this one copies what is left
+    std::memcpy(dst, src, std::min(part, bytes));
+    if (o < bytes) std::memcpy((char *)dst + o, (const char *)src + o, bytes - o);
+    for (auto &t : pool) t.join();
+}
+
+// n host particles into slots dst ..; one outside the box (or at no number) sets *bad
+__global__ void k_put(const double *in, long long n, long long dst, double sx, double sy, long long xl, long long yl,
+                      uint32_t *X, uint32_t *Y, float *VX, float *VY, float *VZ, float *Z, int *bad) {
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+        const double2 *p = reinterpret_cast<const double2 *>(in + 6 * k);
+        const double2 xy = p[0], zu = p[1], vw = p[2];
+        const long long xi = llround(xy.x * sx), yi = llround(xy.y * sy), s = dst + k;
+        if (!(xi >= 0 && xi < xl && yi >= 0 && yi < yl)) *bad = 1;
+        X[s] = (uint32_t)xi; Y[s] = (uint32_t)yi;
+        VX[s] = isnan(zu.y) ? __int_as_float(HOLE_NAN) : (float)zu.y;
+        VY[s] = (float)vw.x; VZ[s] = (float)vw.y;
+        if (Z) Z[s] = (float)zu.x;
+    }
+}
+
+__global__ void k_put_counts(DevCounters *cnt, int sp, long long n) {
+    cnt->n_slots[sp] = n;
+    cnt->n_alive[sp] = n;
+    cnt->n_sorted[sp] = 0;
+    cnt->n_items[sp] = 0;
+}
+
+// Replaces a species' particles.  They go to the buffer that is not in use, which takes over when
+// all of them have been found inside the box: a refused call leaves the species as it was.
+int particles_put(lepic_ctx *c, int sp, const double *vxp, long long n) {
+    SpeciesBuf &B = c->sp[sp];
+    if (n < 0 || n > B.cap) { c->last_err = "particle count exceeds capacity"; return LEPIC_ECAPACITY; }
+    const lepic_config &g = c->cfg;
+    if (n > 0) {
+        IoStage *S;
+        const int r = io_stage(c, n, 1, &S);
+        if (r != LEPIC_OK) return r;
+        const double sx = (double)(1u << c->S) / g.dx, sy = (double)(1u << c->S) / g.dy;
+        const long long xl = (long long)g.nx << c->S, yl = (long long)g.ny << c->S;
+        const int o = 1 - B.cur;
+        LCUDA(cudaMemsetAsync(S->bad, 0, sizeof(int), c->stream));
+        int b = 0;
+        for (long long k = 0; k < n; k += S->cap, b ^= 1) {
+            const long long m = std::min(S->cap, n - k);
+            if (k >= 2 * S->cap) LCUDA(cudaEventSynchronize(S->ev[b]));   // the buffer's last chunk has left it
+            host_copy(S->h[b], vxp + 6 * k, 48 * (size_t)m);
+            LCUDA(cudaMemcpyAsync(S->d[b], S->h[b], 48 * (size_t)m, cudaMemcpyHostToDevice, c->stream));
+            LCUDA(cudaEventRecord(S->ev[b], c->stream));
+            k_put<<<(int)std::min<long long>(div_up(m, 256), c->num_sms * 8), 256, 0, c->stream>>>(
+                S->d[b], m, k, sx, sy, xl, yl, B.X[o], B.Y[o], B.VX[o], B.VY[o], B.VZ[o], B.Z[o], S->bad);
+            LCUDA(cudaGetLastError());
+        }
+        LCUDA(cudaMemcpyAsync(S->hbad, S->bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        LCUDA(cudaStreamSynchronize(c->stream));
+        if (*S->hbad) { c->last_err = "particle outside the box"; return LEPIC_EINVAL; }
+        B.cur = o;
+    }
+    k_put_counts<<<1, 1, 0, c->stream>>>(c->dcnt, sp, n);
+    LCUDA(cudaGetLastError());
+    B.ordered = false;
+    return LEPIC_OK;
+}
+
+// The live particles of a species in slot order (at most cap of them); n_out: how many there are
+int particles_get(lepic_ctx *c, int sp, double *vxp, long long cap, long long *n_out) {
+    int r = lepic_gpu_sync(c);
+    if (r != LEPIC_OK) return r;
+    SpeciesBuf &B = c->sp[sp];
+    const lepic_config &g = c->cfg;
+    const long long ns = c->hcnt->n_slots[sp], nb = div_up(ns, BK_BLOCK);
+    if (n_out) *n_out = 0;
+    if (ns == 0) return LEPIC_OK;
+    IoStage *S;
+    if ((r = io_stage(c, vxp ? ns : 1, nb, &S)) != LEPIC_OK) return r;
+    std::vector<int> cnt((size_t)nb);
+    std::vector<long long> off((size_t)nb + 1, 0);
+    k_live_counts<<<(unsigned)nb, 256, 0, c->stream>>>(B.VX[B.cur], ns, S->counts);
+    LCUDA(cudaGetLastError());
+    LCUDA(cudaMemcpyAsync(cnt.data(), S->counts, sizeof(int) * nb, cudaMemcpyDeviceToHost, c->stream));
+    LCUDA(cudaStreamSynchronize(c->stream));
+    for (long long b = 0; b < nb; b++) off[b + 1] = off[b] + cnt[b];
+    const long long total = off[nb];
+    if (n_out) *n_out = total;
+    if (vxp) {
+        LCUDA(cudaMemcpyAsync(S->off, off.data(), sizeof(long long) * (nb + 1), cudaMemcpyHostToDevice, c->stream));
+        const double ux = g.dx * std::ldexp(1.0, -c->S), uy = g.dy * std::ldexp(1.0, -c->S);
+        const long long per = S->cap / BK_BLOCK;
+        long long at[2] = {0, 0}, len[2] = {0, 0};   // where a buffer's particles go, and how many
+        auto finish = [&](int b) {
+            const cudaError_t e = cudaEventSynchronize(S->ev[b]);
+            if (e == cudaSuccess) host_copy(vxp + 6 * at[b], S->h[b], 48 * (size_t)len[b]);
+            return e;
+        };
+        int b = 0, pending = 0;
+        for (long long b0 = 0; b0 < nb && off[b0] < cap; b0 += per, b ^= 1) {
+            const long long bn = std::min(per, nb - b0);
+            k_pack<<<(unsigned)bn, BK_BLOCK, 0, c->stream>>>(B.X[B.cur], B.Y[B.cur], B.VX[B.cur], B.VY[B.cur], B.VZ[B.cur],
+                                                             B.Z[B.cur], ns, b0, S->off, ux, uy, S->d[b]);
+            LCUDA(cudaGetLastError());
+            at[b] = off[b0];
+            len[b] = std::min(off[b0 + bn], cap) - off[b0];
+            LCUDA(cudaMemcpyAsync(S->h[b], S->d[b], 48 * (size_t)len[b], cudaMemcpyDeviceToHost, c->stream));
+            LCUDA(cudaEventRecord(S->ev[b], c->stream));
+            if (pending) LCUDA(finish(b ^ 1));       // the chunk before, while this one is on its way
+            pending = 1;
+        }
+        if (pending) LCUDA(finish(b ^ 1));
+    }
+    if (vxp && total > cap) { c->last_err = "output capacity too small"; return LEPIC_ECAPACITY; }
+    return LEPIC_OK;
 }
 
 // ---------------------------------------------------------------------------------------

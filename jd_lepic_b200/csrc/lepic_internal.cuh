@@ -243,6 +243,8 @@ struct lepic_ctx {
     int ev_cap = 0;
     double Ca = 0.0;
     double *dq = nullptr;
+    // staging of particles between the host's FP64 array and the device (backup.cu)
+    void *io = nullptr;
     // particle sources (sources.cu), created by lepic_gpu_set_sources
     void *src = nullptr;
     // averaging diagnostics (diag.cu), created by lepic_gpu_set_avg
@@ -454,6 +456,7 @@ int wait_upload(lepic_ctx *c);
 bool push_needs_general(const lepic_ctx *c, int s);
 int particles_load(lepic_ctx *c, const lepic_load_spec *spec);
 int particles_put(lepic_ctx *c, int ptype, const double *vxp, long long n);
+void io_free(lepic_ctx *c);
 int particles_get(lepic_ctx *c, int ptype, double *vxp, long long cap, long long *n_out);
 int sources_before_push(lepic_ctx *c, int it);
 int sources_after_push(lepic_ctx *c, int it);
