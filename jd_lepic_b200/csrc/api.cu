@@ -122,8 +122,7 @@ static int create_impl(lepic_ctx *c, const lepic_config *cfg, const int32_t *bcn
             cw[ix + (size_t)iy * (nx + 2)] = wall ? 1 : 0;
             cww[ix + (size_t)iy * W] = wall ? 1 : 0;
         }
-    // the masks are 16 bytes longer: the mixed solver's tiles read them in whole words
-    LALLOC(c->bcnd, nn); LALLOC(c->bc8, nn + 16); LALLOC(c->cellwall, cw.size()); LALLOC(c->cellwall_w, cww.size()); LALLOC(c->kq, nn);
+    LALLOC(c->bcnd, nn); LALLOC(c->bc8, nn); LALLOC(c->cellwall, cw.size()); LALLOC(c->cellwall_w, cww.size()); LALLOC(c->kq, nn);
     LCUDA(cudaMemcpy(c->bcnd, bcnd, sizeof(int32_t) * nn, cudaMemcpyHostToDevice));
     LCUDA(cudaMemcpy(c->bc8, bc8.data(), nn, cudaMemcpyHostToDevice));
     LCUDA(cudaMemcpy(c->cellwall, cw.data(), cw.size(), cudaMemcpyHostToDevice));
@@ -206,7 +205,7 @@ static int create_impl(lepic_ctx *c, const lepic_config *cfg, const int32_t *bcn
             cur[L.nx + 2] = prev[nxf + 2];
             cur[(L.ny + 2) * W2] = prev[(nyf + 2) * Wf];
             cur[L.nx + 2 + (L.ny + 2) * W2] = prev[nxf + 2 + (nyf + 2) * Wf];
-            LALLOC(L.u, nnl); LALLOC(L.u2, nnl + L.ny + 3); LALLOC(L.b, (size_t)(L.nx + 1) * (L.ny + 1)); LALLOC(L.bc, nnl + 16);
+            LALLOC(L.u, nnl); LALLOC(L.u2, nnl + L.ny + 3); LALLOC(L.b, (size_t)(L.nx + 1) * (L.ny + 1)); LALLOC(L.bc, nnl);
             LCUDA(cudaMemset(L.u, 0, sizeof(double) * nnl));
             LCUDA(cudaMemset(L.b, 0, sizeof(double) * (L.nx + 1) * (L.ny + 1)));
             LCUDA(cudaMemcpy(L.bc, cur.data(), nnl, cudaMemcpyHostToDevice));
