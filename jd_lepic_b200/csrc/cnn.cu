@@ -392,7 +392,10 @@ __global__ void __launch_bounds__(CONV_THREADS, (CIN == 16 && COUT == 16) ? 10 :
 
 // ---------------------------------------------------------------------------------------
 // weight gradient on the CUDA cores: dW[n][c][tap] = sum_p G[p][n] * X[p + tap][c] per work
-// unit (image, strip, R rows) into per-unit partials, reduced in unit order afterwards
+// unit (image, strip, R rows) into per-unit partials, reduced in unit order afterwards.  Bound by
+// its shared-memory loads (two per 16 products); a strip narrower than 128 pixels (the deeper
+// levels' whole rows) is walked only as far as it goes (64 -> 64 channels at crops of 32 and 16
+// pixels: 43 -> 19 us per launch).
 struct DwP {
     ConvP X;              // the convolution input as the forward pass read it (in, in_mode, sizes)
     const bf16 *G;        // output gradient [N][H][W][COUT]
@@ -415,6 +418,7 @@ __global__ void __launch_bounds__(DW_THREADS) k_conv_dw(DwP D) {
     const int rem = u - n * nstrip * nrb;
     const int rb = rem / nstrip, xs = rem - rb * nstrip;
     const int x0 = xs * 128, y0 = rb * P.R, y1 = min(y0 + P.R, P.H);
+    const int mw = min(128, P.W - x0);     // pixels of the strip
     const int widx = blockIdx.y * DW_THREADS + tid;
     const bool active = widx < NBLK;
     const int tap = active ? widx / (NB * CB) : 0;
@@ -433,19 +437,15 @@ __global__ void __launch_bounds__(DW_THREADS) k_conv_dw(DwP D) {
     for (int y = y0; y < y1; y++) {
         load_row<CIN, DW_THREADS>(P, s_in, n, y + 1, x0, (y + 2) & 3);
         cp_async_commit();
-        for (int i = tid; i < 128 * (COUT / 8); i += DW_THREADS) {
-            const int p = i / (COUT / 8), c8 = i - p * (COUT / 8);
-            const int xx = x0 + p;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (xx < P.W) v = __ldg(reinterpret_cast<const uint4 *>(D.G + (((size_t)n * P.H + y) * P.W + xx) * COUT) + c8);
-            reinterpret_cast<uint4 *>(s_g)[i] = v;
-        }
+        const uint4 *gr = reinterpret_cast<const uint4 *>(D.G + (((size_t)n * P.H + y) * P.W + x0) * COUT);
+        for (int i = tid; i < mw * (COUT / 8); i += DW_THREADS) reinterpret_cast<uint4 *>(s_g)[i] = __ldg(gr + i);
         cp_async_wait_all();
         __syncthreads();
         if (active) {
             const int slot = (y + dy) & 3;
             const unsigned char *xb = s_in + ((size_t)(slot * NCH + (cb >> 1)) * CONV_PITCH + dx) * 16 + (cb & 1) * 8;
-            for (int m = 0; m < 128; m++) {
+#pragma unroll 4
+            for (int m = 0; m < mw; m++) {
                 const uint2 gq = *reinterpret_cast<const uint2 *>(s_g + m * COUT + nb * 4);
                 const uint2 xq = *reinterpret_cast<const uint2 *>(xb + m * 16);
                 const float2 g01 = bf2_to_f2(gq.x), g23 = bf2_to_f2(gq.y);
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(DW_THREADS) k_conv_dw(DwP D) {
             }
         }
         if (bias_thr)
-            for (int m = 0; m < 128; m++) db += __bfloat162float(s_g[m * COUT + tid]);
+            for (int m = 0; m < mw; m++) db += __bfloat162float(s_g[m * COUT + tid]);
         __syncthreads();
     }
     if (active) {
