@@ -3,8 +3,8 @@
 // MOD(it,navg) == 1 (main.f90:906-949).  data_pavg and phi_avg stay on the device in the
 // reference's Fortran layouts; the host reads them when it writes its files.
 //
-// k_moments: one particle per thread in slot order (the particles are cell-sorted at this
-// step, main.f90:891-906): the back-stepped position xp = x - vx dt/2 selects a cell of the
+// k_moments: eight consecutive particles per thread in slot order (the particles are cell-sorted at
+// this step, main.f90:891-906): the back-stepped position xp = x - vx dt/2 selects a cell of the
 // coarse grid (size_na cells of the field grid per cell); the 16 contributions (4 nodes x
 // n<v^2>, jx, jy, jz) of lanes that share a cell are combined by a segmented warp scan and the
 // last lane of each segment adds them with FP64 atomics.  FP64 sums in atomic order: the
@@ -79,19 +79,48 @@ __device__ __forceinline__ int moment_of(const MomP &P, long long k, double *c) 
     return ix + iy * (P.na1 + 3);
 }
 
+// 16 sums of one coarse cell added to its four nodes
+__device__ __forceinline__ void add_moments(const MomP &P, int key, const double *c) {
+    const int ix = key % (P.na1 + 3), iy = key / (P.na1 + 3);
+    const long long nodes[4] = {ix + (long long)iy * (P.na1 + 3), ix + 1 + (long long)iy * (P.na1 + 3),
+                                ix + 1 + (long long)(iy + 1) * (P.na1 + 3), ix + (long long)(iy + 1) * (P.na1 + 3)};
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+            if (c[4 * q + m] != 0.0) atomicAdd(P.p_mts + m * P.ncell + nodes[q], c[4 * q + m]);
+}
+
+// Each thread first sums MOM_G consecutive slots while they stay in one coarse cell (a run that
+// ends inside is added at once), then the warp combines its lanes' runs: bound by the 160
+// shuffles of that scan, which one particle per lane paid 8 times as often (2 x 5.9 M particles
+// on 384 x 256 cells: 0.48 ms per sample; the whole 10-step pass with two samples 16.2 -> 15.9 ms).
+#define MOM_G 8
 __global__ void __launch_bounds__(256) k_moments(MomP P) {
     const long long n = P.cnt->n_slots[P.sp];
     const int lane = threadIdx.x & 31;
     const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
     const long long w0 = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
-    for (long long base = w0 * 32; base < n; base += nwarps * 32) {   // warp-uniform trip count
-        const long long k = base + lane;
+    for (long long base = w0 * (32 * MOM_G); base < n; base += nwarps * (32 * MOM_G)) {   // warp-uniform trip count
         double c[16];
         int key = -1;
-        if (k < n) key = moment_of(P, k, c);
-        if (key < 0) {
 #pragma unroll
-            for (int q = 0; q < 16; q++) c[q] = 0.0;
+        for (int q = 0; q < 16; q++) c[q] = 0.0;
+        for (int p = 0; p < MOM_G; p++) {
+            const long long k = base + (long long)lane * MOM_G + p;
+            if (k >= n) break;
+            double d[16];
+            const int kk = moment_of(P, k, d);
+            if (kk < 0) continue;
+            if (kk != key) {
+                if (key >= 0) add_moments(P, key, c);
+                key = kk;
+#pragma unroll
+                for (int q = 0; q < 16; q++) c[q] = d[q];
+            } else {
+#pragma unroll
+                for (int q = 0; q < 16; q++) c[q] += d[q];
+            }
         }
         // segmented inclusive scan: a segment is a run of equal keys in lane order (one run
         // per cell after the sort); segment ids from the run heads keep runs of a key that
@@ -110,17 +139,7 @@ __global__ void __launch_bounds__(256) k_moments(MomP P) {
             }
         }
         const bool last = lane == 31 || ((heads >> (lane + 1)) & 1u);
-        if (key >= 0 && last) {
-            const int ix = key % (P.na1 + 3), iy = key / (P.na1 + 3);
-            const long long nodes[4] = {ix + (long long)iy * (P.na1 + 3), ix + 1 + (long long)iy * (P.na1 + 3),
-                                        ix + 1 + (long long)(iy + 1) * (P.na1 + 3),
-                                        ix + (long long)(iy + 1) * (P.na1 + 3)};
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-#pragma unroll
-                for (int m = 0; m < 4; m++)
-                    if (c[4 * q + m] != 0.0) atomicAdd(P.p_mts + m * P.ncell + nodes[q], c[4 * q + m]);
-        }
+        if (key >= 0 && last) add_moments(P, key, c);
     }
 }
 
