@@ -120,8 +120,4 @@ __device__ __forceinline__ bool team_sums(const BigTeam &T, const double (&v)[N]
     __syncthreads();
     return true;
 }
-__device__ __forceinline__ bool team_sum(const SmallTeam &, double v, double *out) {
-    *out = block_sum(v);
-    return true;
-}
 
