@@ -173,6 +173,8 @@ static int create_impl(lepic_ctx *c, const lepic_config *cfg, const int32_t *bcn
         B.prod_cap = (int)std::min<long long>(1 << 24, std::max<long long>(65536, B.cap / 50));
         LALLOC(B.prod, B.prod_cap);
     }
+    // keys and perm also stage particles between host and device (backup.cu)
+    maxcap = std::max(maxcap, (long long)IO_MIN_SCRATCH);
     c->scratch_cap = maxcap;
     LALLOC(c->keys, maxcap); LALLOC(c->perm, maxcap);
     LALLOC(c->counts, c->nkeys + 1); LALLOC(c->offsets, c->nkeys + 1); LALLOC(c->cursor, c->nkeys + 1);

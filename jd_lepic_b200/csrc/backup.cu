@@ -96,81 +96,55 @@ __global__ void k_unpack(const double *in, long long n, long long dst, double sx
 }
 
 // ---------------------------------------------------------------------------------------
-// Particles to and from the host's FP64 vxp(6, n): the records cross in chunks of IO_CHUNK through
-// two pinned buffers, the conversion to and from the device's arrays is done on the device, and
-// each chunk's host copy (by a few threads: one thread's copy, and its page faults on a new array,
-// are slower than the bus) runs beside the transfer and conversion of the other.  Bound by those
-// host copies: 48 B per particle each way.  (Converted by one host thread between plain copies,
-// put + sort + deposit + get of 2 x 1.3 M particles took 67 ms; so 22 ms, most of it
-// the page faults of the fresh host arrays.)
-#define IO_CHUNK (1ll << 17)          // particles per chunk (a multiple of BK_BLOCK): 6.3 MB
+// Particles to and from the host's FP64 vxp(6, n): the records cross in chunks, converted to and
+// from the device's arrays on the device.  The device side of a chunk is the sort's scratch (keys
+// and perm, free between sorts), taken in turns.  From IO_PINNED particles on, the host side goes
+// through two pinned buffers, filled or emptied by a few threads (one thread's copy, and its page
+// faults on a new array, are slower than the bus) beside the transfer and conversion of the
+// other chunk; fewer cross straight from and to the caller's array, since pinning the buffers at a
+// context's first call costs about 10 ms, more than it then saves.  (Converted by one host thread
+// between plain copies, put + sort + deposit + get of 2 x 1.3 M particles took 66 ms; so 21 ms, most
+// of it the page faults of the fresh host arrays.)
+#define IO_CHUNK (1ll << 17)          // particles per chunk at most (a multiple of BK_BLOCK): 6.3 MB (2^16: 31 ms)
+#define IO_PINNED (1ll << 19)
 struct IoStage {
-    long long cap = 0;                // particles per buffer
-    double *d[2] = {nullptr, nullptr}, *h[2] = {nullptr, nullptr};
+    double *h[2] = {nullptr, nullptr};
     cudaEvent_t ev[2] = {nullptr, nullptr};
-    long long blocks = 0;             // entries of the two below
-    int *counts = nullptr;
-    long long *off = nullptr;
-    int *bad = nullptr;               // a particle outside the box (device), and its pinned mirror
-    int *hbad = nullptr;
 };
 
 void io_free(lepic_ctx *c) {
     IoStage *S = (IoStage *)c->io;
     if (!S) return;
     for (int k = 0; k < 2; k++) {
-        if (S->d[k]) cudaFree(S->d[k]);
         if (S->h[k]) cudaFreeHost(S->h[k]);
         if (S->ev[k]) cudaEventDestroy(S->ev[k]);
     }
-    if (S->counts) cudaFree(S->counts);
-    if (S->off) cudaFree(S->off);
-    if (S->bad) cudaFree(S->bad);
-    if (S->hbad) cudaFreeHost(S->hbad);
     delete S;
     c->io = nullptr;
 }
 
-// the context's staging for n particles (at most IO_CHUNK at a time) and nb counting blocks; kept
-// until the context is destroyed
-static int io_stage(lepic_ctx *c, long long n, long long nb, IoStage **out) {
-    if (!c->io) c->io = new (std::nothrow) IoStage;
-    IoStage *S = (IoStage *)c->io;
-    if (!S) { c->last_err = "particle staging: out of host memory"; return LEPIC_ENOMEM; }
-    auto fail = [&](cudaError_t e) {
-        c->last_err = std::string("particle staging: ") + cudaGetErrorString(e);
-        io_free(c);
-        return LEPIC_ENOMEM;
-    };
-    cudaError_t e;
-    if (!S->bad) {
-        if ((e = cudaMalloc((void **)&S->bad, sizeof(int))) != cudaSuccess) return fail(e);
-        if ((e = cudaMallocHost((void **)&S->hbad, sizeof(int))) != cudaSuccess) return fail(e);
-        for (int k = 0; k < 2; k++)
-            if ((e = cudaEventCreateWithFlags(&S->ev[k], cudaEventDisableTiming)) != cudaSuccess) return fail(e);
-    }
-    const long long want = std::min(IO_CHUNK, (n + BK_BLOCK - 1) / BK_BLOCK * BK_BLOCK);
-    if (S->cap < want) {
-        S->cap = 0;
-        for (int k = 0; k < 2; k++) {
-            if (S->d[k]) cudaFree(S->d[k]);
-            if (S->h[k]) cudaFreeHost(S->h[k]);
-            S->d[k] = S->h[k] = nullptr;
-            if ((e = cudaMalloc((void **)&S->d[k], 48 * want)) != cudaSuccess) return fail(e);
-            if ((e = cudaMallocHost((void **)&S->h[k], 48 * want)) != cudaSuccess) return fail(e);
+// the context's pinned buffers, kept until it is destroyed; null when they cannot be had (the
+// caller's array is then used directly)
+static IoStage *io_stage(lepic_ctx *c) {
+    if (c->io) return (IoStage *)c->io;
+    IoStage *S = new (std::nothrow) IoStage;
+    if (!S) return nullptr;
+    c->io = S;
+    for (int k = 0; k < 2; k++)
+        if (cudaMallocHost((void **)&S->h[k], 48 * IO_CHUNK) != cudaSuccess ||
+            cudaEventCreateWithFlags(&S->ev[k], cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            io_free(c);
+            return nullptr;
         }
-        S->cap = want;
-    }
-    if (S->blocks < nb) {
-        if (S->counts) cudaFree(S->counts);
-        if (S->off) cudaFree(S->off);
-        S->counts = nullptr; S->off = nullptr; S->blocks = 0;
-        if ((e = cudaMalloc((void **)&S->counts, sizeof(int) * nb)) != cudaSuccess) return fail(e);
-        if ((e = cudaMalloc((void **)&S->off, sizeof(long long) * (nb + 1))) != cudaSuccess) return fail(e);
-        S->blocks = nb;
-    }
-    *out = S;
-    return LEPIC_OK;
+    return S;
+}
+
+// particles per chunk, a multiple of BK_BLOCK, behind `used` bytes of the scratch (which holds at
+// least one such block: IO_MIN_SCRATCH)
+static long long io_chunk(const lepic_ctx *c, long long used) {
+    const long long per = (4 * c->scratch_cap - used) / 48 / BK_BLOCK * BK_BLOCK;
+    return std::min(IO_CHUNK, per);
 }
 
 // memcpy by up to four threads
@@ -222,27 +196,33 @@ int particles_put(lepic_ctx *c, int sp, const double *vxp, long long n) {
     if (n < 0 || n > B.cap) { c->last_err = "particle count exceeds capacity"; return LEPIC_ECAPACITY; }
     const lepic_config &g = c->cfg;
     if (n > 0) {
-        IoStage *S;
-        const int r = io_stage(c, n, 1, &S);
-        if (r != LEPIC_OK) return r;
+        IoStage *S = n >= IO_PINNED ? io_stage(c) : nullptr;
         const double sx = (double)(1u << c->S) / g.dx, sy = (double)(1u << c->S) / g.dy;
         const long long xl = (long long)g.nx << c->S, yl = (long long)g.ny << c->S;
+        const long long chunk = io_chunk(c, 0);
+        double *const d[2] = {(double *)c->keys, (double *)c->perm};
+        int *const bad = c->blocksums;                   // scratch of the sort's scan
         const int o = 1 - B.cur;
-        LCUDA(cudaMemsetAsync(S->bad, 0, sizeof(int), c->stream));
+        LCUDA(cudaMemsetAsync(bad, 0, sizeof(int), c->stream));
         int b = 0;
-        for (long long k = 0; k < n; k += S->cap, b ^= 1) {
-            const long long m = std::min(S->cap, n - k);
-            if (k >= 2 * S->cap) LCUDA(cudaEventSynchronize(S->ev[b]));   // the buffer's last chunk has left it
-            host_copy(S->h[b], vxp + 6 * k, 48 * (size_t)m);
-            LCUDA(cudaMemcpyAsync(S->d[b], S->h[b], 48 * (size_t)m, cudaMemcpyHostToDevice, c->stream));
-            LCUDA(cudaEventRecord(S->ev[b], c->stream));
+        for (long long k = 0; k < n; k += chunk, b ^= 1) {
+            const long long m = std::min(chunk, n - k);
+            const double *src = vxp + 6 * k;
+            if (S) {
+                if (k >= 2 * chunk) LCUDA(cudaEventSynchronize(S->ev[b]));   // the buffer's last chunk has left it
+                host_copy(S->h[b], src, 48 * (size_t)m);
+                src = S->h[b];
+            }
+            LCUDA(cudaMemcpyAsync(d[b], src, 48 * (size_t)m, cudaMemcpyHostToDevice, c->stream));
+            if (S) LCUDA(cudaEventRecord(S->ev[b], c->stream));
             k_put<<<(int)std::min<long long>(div_up(m, 256), c->num_sms * 8), 256, 0, c->stream>>>(
-                S->d[b], m, k, sx, sy, xl, yl, B.X[o], B.Y[o], B.VX[o], B.VY[o], B.VZ[o], B.Z[o], S->bad);
+                d[b], m, k, sx, sy, xl, yl, B.X[o], B.Y[o], B.VX[o], B.VY[o], B.VZ[o], B.Z[o], bad);
             LCUDA(cudaGetLastError());
         }
-        LCUDA(cudaMemcpyAsync(S->hbad, S->bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        int hbad = 0;
+        LCUDA(cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
         LCUDA(cudaStreamSynchronize(c->stream));
-        if (*S->hbad) { c->last_err = "particle outside the box"; return LEPIC_EINVAL; }
+        if (hbad) { c->last_err = "particle outside the box"; return LEPIC_EINVAL; }
         B.cur = o;
     }
     k_put_counts<<<1, 1, 0, c->stream>>>(c->dcnt, sp, n);
@@ -260,21 +240,25 @@ int particles_get(lepic_ctx *c, int sp, double *vxp, long long cap, long long *n
     const long long ns = c->hcnt->n_slots[sp], nb = div_up(ns, BK_BLOCK);
     if (n_out) *n_out = 0;
     if (ns == 0) return LEPIC_OK;
-    IoStage *S;
-    if ((r = io_stage(c, vxp ? ns : 1, nb, &S)) != LEPIC_OK) return r;
+    // the scratch: block offsets and counts at the start of keys, then one chunk; perm the other
+    const long long used = (8 * (nb + 1) + 4 * nb + 255) / 256 * 256;
+    long long *const d_off = (long long *)c->keys;
+    int *const d_cnt = (int *)(d_off + nb + 1);
+    double *const d[2] = {(double *)((char *)c->keys + used), (double *)c->perm};
     std::vector<int> cnt((size_t)nb);
     std::vector<long long> off((size_t)nb + 1, 0);
-    k_live_counts<<<(unsigned)nb, 256, 0, c->stream>>>(B.VX[B.cur], ns, S->counts);
+    k_live_counts<<<(unsigned)nb, 256, 0, c->stream>>>(B.VX[B.cur], ns, d_cnt);
     LCUDA(cudaGetLastError());
-    LCUDA(cudaMemcpyAsync(cnt.data(), S->counts, sizeof(int) * nb, cudaMemcpyDeviceToHost, c->stream));
+    LCUDA(cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(int) * nb, cudaMemcpyDeviceToHost, c->stream));
     LCUDA(cudaStreamSynchronize(c->stream));
     for (long long b = 0; b < nb; b++) off[b + 1] = off[b] + cnt[b];
     const long long total = off[nb];
     if (n_out) *n_out = total;
     if (vxp) {
-        LCUDA(cudaMemcpyAsync(S->off, off.data(), sizeof(long long) * (nb + 1), cudaMemcpyHostToDevice, c->stream));
+        IoStage *S = total >= IO_PINNED ? io_stage(c) : nullptr;
+        LCUDA(cudaMemcpyAsync(d_off, off.data(), sizeof(long long) * (nb + 1), cudaMemcpyHostToDevice, c->stream));
         const double ux = g.dx * std::ldexp(1.0, -c->S), uy = g.dy * std::ldexp(1.0, -c->S);
-        const long long per = S->cap / BK_BLOCK;
+        const long long per = io_chunk(c, used) / BK_BLOCK;
         long long at[2] = {0, 0}, len[2] = {0, 0};   // where a buffer's particles go, and how many
         auto finish = [&](int b) {
             const cudaError_t e = cudaEventSynchronize(S->ev[b]);
@@ -285,16 +269,18 @@ int particles_get(lepic_ctx *c, int sp, double *vxp, long long cap, long long *n
         for (long long b0 = 0; b0 < nb && off[b0] < cap; b0 += per, b ^= 1) {
             const long long bn = std::min(per, nb - b0);
             k_pack<<<(unsigned)bn, BK_BLOCK, 0, c->stream>>>(B.X[B.cur], B.Y[B.cur], B.VX[B.cur], B.VY[B.cur], B.VZ[B.cur],
-                                                             B.Z[B.cur], ns, b0, S->off, ux, uy, S->d[b]);
+                                                             B.Z[B.cur], ns, b0, d_off, ux, uy, d[b]);
             LCUDA(cudaGetLastError());
             at[b] = off[b0];
             len[b] = std::min(off[b0 + bn], cap) - off[b0];
-            LCUDA(cudaMemcpyAsync(S->h[b], S->d[b], 48 * (size_t)len[b], cudaMemcpyDeviceToHost, c->stream));
+            LCUDA(cudaMemcpyAsync(S ? S->h[b] : vxp + 6 * at[b], d[b], 48 * (size_t)len[b], cudaMemcpyDeviceToHost, c->stream));
+            if (!S) continue;
             LCUDA(cudaEventRecord(S->ev[b], c->stream));
             if (pending) LCUDA(finish(b ^ 1));       // the chunk before, while this one is on its way
             pending = 1;
         }
         if (pending) LCUDA(finish(b ^ 1));
+        else LCUDA(cudaStreamSynchronize(c->stream));
     }
     if (vxp && total > cap) { c->last_err = "output capacity too small"; return LEPIC_ECAPACITY; }
     return LEPIC_OK;

@@ -243,7 +243,7 @@ struct lepic_ctx {
     int ev_cap = 0;
     double Ca = 0.0;
     double *dq = nullptr;
-    // staging of particles between the host's FP64 array and the device (backup.cu)
+    // pinned staging of particles between the host's FP64 array and the device (backup.cu)
     void *io = nullptr;
     // particle sources (sources.cu), created by lepic_gpu_set_sources
     void *src = nullptr;
@@ -315,11 +315,6 @@ __device__ __forceinline__ void set_err(DevCounters *c, int bit, int where) {
 
 // Bounded software grid barrier for cooperative launches.  Every wait gives up after a
 // clock budget (about 2 s) and then raises LERR_TIMEOUT; any raised error ends all waits.
-__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p) {
-    unsigned int v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 __device__ __forceinline__ int ld_volatile_i32(const int *p) {
     int v;
     asm volatile("ld.volatile.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -334,7 +329,8 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
 // the arrivals of barrier k are the values k nblocks .. (k + 1) nblocks - 1 (no CTA arrives at
 // barrier k + 1 before barrier k is complete), so a CTA reads its barrier from the value its
 // atomic returns and waits until the counter reaches the end of that barrier.  With no reset
-// between barriers one atomic and one acquire poll are on the critical path (1.8 us per
+// between barriers one atomic and one poll (relaxed; the fence behind it orders what follows) are
+// on the critical path (1.8 us per
 // barrier over 444 CTAs on B200, against 2.8 us for a count-and-generation barrier, measured
 // by a standalone probe).
 __device__ __forceinline__ bool grid_barrier(DevCounters *c, unsigned int nblocks) {
@@ -457,6 +453,7 @@ bool push_needs_general(const lepic_ctx *c, int s);
 int particles_load(lepic_ctx *c, const lepic_load_spec *spec);
 int particles_put(lepic_ctx *c, int ptype, const double *vxp, long long n);
 void io_free(lepic_ctx *c);
+#define IO_MIN_SCRATCH 16384   // ints: a block of 1024 particles at 48 B, and its offsets
 int particles_get(lepic_ctx *c, int ptype, double *vxp, long long cap, long long *n_out);
 int sources_before_push(lepic_ctx *c, int it);
 int sources_after_push(lepic_ctx *c, int it);

@@ -10,7 +10,7 @@ from jd_lepic_b200 import _capi as capi, configs
 
 pytestmark = pytest.mark.gpu
 
-CHUNK = 131072
+CHUNK = 131072     # the largest chunk; pinned buffers from 4 of them on
 
 
 def _particles(case, n, seed):
@@ -32,7 +32,7 @@ def _stored(p, case):
     return q
 
 
-@pytest.mark.parametrize("n", [0, 1, 1023, CHUNK - 1, CHUNK, CHUNK + 1, 2 * CHUNK + 5, 5 * CHUNK - 700])
+@pytest.mark.parametrize("n", [0, 1, 1023, CHUNK - 1, CHUNK, CHUNK + 1, 2 * CHUNK + 5, 5 * CHUNK - 700, 6 * CHUNK + 3])
 def test_round_trip(gpu_lib, n):
     from jd_lepic_b200.simulation import GpuSimulation
     case = configs.case0(ppc=1, nx=64, ny=48)
@@ -63,12 +63,13 @@ def test_round_trip(gpu_lib, n):
         s.close()
 
 
+@pytest.mark.parametrize("size", [2, 4])
 @pytest.mark.parametrize("at", [0, CHUNK - 1, 2 * CHUNK + 3])
 @pytest.mark.parametrize("what", [(0, -1e-4), (1, 1.0), (0, np.nan), (1, np.inf)])
-def test_refused_put_changes_nothing(gpu_lib, at, what):
+def test_refused_put_changes_nothing(gpu_lib, at, what, size):
     from jd_lepic_b200.simulation import GpuSimulation
     case = configs.case0(ppc=1, nx=32, ny=32)
-    n = 2 * CHUNK + 10
+    n = size * CHUNK + 10
     s = GpuSimulation(case, tile=(8, 8), load=False, capacity=n)
     try:
         p = _particles(case, 5000, 1)
