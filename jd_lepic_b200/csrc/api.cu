@@ -207,7 +207,8 @@ static int create_impl(lepic_ctx *c, const lepic_config *cfg, const int32_t *bcn
             cur[L.nx + 2] = prev[nxf + 2];
             cur[(L.ny + 2) * W2] = prev[(nyf + 2) * Wf];
             cur[L.nx + 2 + (L.ny + 2) * W2] = prev[nxf + 2 + (nyf + 2) * Wf];
-            LALLOC(L.u, nnl); LALLOC(L.u2, nnl + L.ny + 3); LALLOC(L.b, (size_t)(L.nx + 1) * (L.ny + 1)); LALLOC(L.bc, nnl);
+            L.u2_len = mg_level_len(L.nx, L.ny);
+            LALLOC(L.u, nnl); LALLOC(L.u2, (size_t)L.u2_len); LALLOC(L.b, (size_t)(L.nx + 1) * (L.ny + 1)); LALLOC(L.bc, nnl);
             LCUDA(cudaMemset(L.u, 0, sizeof(double) * nnl));
             LCUDA(cudaMemset(L.b, 0, sizeof(double) * (L.nx + 1) * (L.ny + 1)));
             LCUDA(cudaMemcpy(L.bc, cur.data(), nnl, cudaMemcpyHostToDevice));
@@ -221,8 +222,9 @@ static int create_impl(lepic_ctx *c, const lepic_config *cfg, const int32_t *bcn
     // grid-wide sums: up to 3 values x 2 halves per CTA of a cooperative grid of at most 8 CTAs
     // of 256 threads per SM
     LALLOC(c->partials, (size_t)c->num_sms * 48);
-    // cg_ap: also the FP64 multigrid's second level-0 buffer, whose rows may be one node longer
-    LALLOC(c->cg_r, nn); LALLOC(c->cg_p, nn); LALLOC(c->cg_ap, nn + ny + 3);
+    // cg_ap: also the FP64 multigrid's second level-0 buffer
+    c->lev[0].u2_len = mg_level_len(nx, ny);
+    LALLOC(c->cg_r, nn); LALLOC(c->cg_p, nn); LALLOC(c->cg_ap, (size_t)c->lev[0].u2_len);
     LCUDA(cudaMemset(c->cg_r, 0, sizeof(double) * nn));
     LCUDA(cudaMemset(c->cg_p, 0, sizeof(double) * nn));
     LCUDA(cudaMemset(c->cg_ap, 0, sizeof(double) * nn));

@@ -14,6 +14,7 @@
 #include <stdint.h>
 #include <string>
 #include "../../include/lepic_gpu.h"
+#include "mg_layout.h"
 
 #define LEPIC_DEP_SHIFT 44          // deposit fixed point: weight * 2^44
 #define LEPIC_MAXLEV 16
@@ -108,7 +109,8 @@ struct MGLevel {
     int nx, ny;
     double hx, hy;
     double *u;       // (nx+3)(ny+3)
-    double *u2;      // the FP64 multigrid's second buffer (level 0 uses the CG vector cg_ap)
+    double *u2;      // the FP64 multigrid's second buffer (level 0: the CG vector cg_ap)
+    long long u2_len;   // its length: mg_level_len() or more
     double *b;       // (nx+1)(ny+1)
     int8_t *bc;      // (nx+3)(ny+3), bcnd clamped to [-4, 1]
     float *e32;      // mixed precision correction (nx+3)(ny+3)

@@ -110,7 +110,7 @@ __device__ __forceinline__ Patch tile_patch(const MGP &P, const MGDev &L, int ti
     g.j1 = min(g.j0 + TY, ny + 2);
     g.ri0 = max(g.i0 - H, 0);
     g.RW = min(g.i1 + H, nx + 3) - g.ri0;
-    g.RP = g.RW | 1;
+    g.RP = mg_pitch(g.RW);
     g.wrap = 0; g.nA = g.n0 = 0; g.a0 = 0;
     g.b0 = max(g.j0 - H, 0);
     g.RH = min(g.j1 + H, ny + 3) - g.b0;
@@ -132,7 +132,7 @@ __device__ __forceinline__ Patch tile_patch(const MGP &P, const MGDev &L, int ti
         }
     }
     g.par = (g.ri0 + (g.nA ? g.a0 : g.b0)) & 1;
-    g.PS = (g.RP * g.RH + 1) >> 1;
+    g.PS = mg_plane(g.RP, g.RH);
     g.uo = MG_SLOTS;
     g.bo = MG_SLOTS + P.cap;
     g.mo = 8 * (MG_SLOTS + 2 * P.cap);
@@ -150,12 +150,12 @@ __device__ __forceinline__ Patch level_patch(const MGP &P, int l) {
     Patch g;
     g.nx = L.nx; g.ny = L.ny;
     g.i0 = 1; g.i1 = L.nx + 2; g.j0 = 1; g.j1 = L.ny + 2;
-    g.ri0 = 0; g.RW = L.nx + 3; g.RP = g.RW | 1; g.RH = L.ny + 3;
+    g.ri0 = 0; g.RW = L.nx + 3; g.RP = mg_pitch(g.RW); g.RH = L.ny + 3;
     g.nA = g.n0 = 0; g.a0 = 0; g.b0 = 0;
     g.clip0 = g.clip1 = CLIP_ALL;
     g.par = 0;
     g.wrap = P.pbc ? 3 : 0;
-    g.PS = (g.RP * g.RH + 1) >> 1;
+    g.PS = mg_plane(g.RP, g.RH);
     g.uo = MG_SLOTS + L.su;
     g.bo = MG_SLOTS + L.sb;
     g.mo = 8 * MG_SLOTS + L.sm;
@@ -881,7 +881,7 @@ static MGP mg_params(lepic_ctx *c, double eps, int mode) {
     const long long room = MG_SMEM / 8 - MG_SLOTS;      // doubles
     long long total = 0;                                // nodes of the CTA-0 part, both colours' padding included
     P.Ls = c->nlev;
-    auto padded = [&](int l) { return ((long long)((c->lev[l].nx + 3) | 1) * (c->lev[l].ny + 3) + 2) / 2 * 2; };
+    auto padded = [&](int l) { return mg_level_len(c->lev[l].nx, c->lev[l].ny); };
     for (int l = c->nlev - 1; l >= 0; l--) {
         const MGLevel &a = c->lev[l];
         if ((long long)(a.nx + 1) * (a.ny + 1) > small_nodes || padded(l) > MG_SLOTS ||
@@ -937,6 +937,11 @@ int mg_init(lepic_ctx *c) {
 
 int mg_solve(lepic_ctx *c, double eps, int mode) {
     MGP P = mg_params(c, eps, mode);
+    for (int l = P.Ls; l < P.ng; l++)
+        if (c->lev[l].u2_len < mg_level_len(P.L[l].nx, P.L[l].ny)) {   // a stage keeps its start there
+            c->last_err = "multigrid: a level's second buffer is too short";
+            return LEPIC_ECUDA;
+        }
     void *args[] = {&P};
     LCUDA(cudaMemsetAsync(&c->dcnt->bar_arrived, 0, sizeof(unsigned long long) + sizeof(int), c->stream));
     LCUDA(cudaLaunchCooperativeKernel((void *)k_mg_solve, dim3(P.Ls == 0 ? 1 : c->mg_grid), dim3(MGT), args, MG_SMEM, c->stream));

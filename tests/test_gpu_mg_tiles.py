@@ -36,7 +36,9 @@ def _case(nx, ny, ng, kind):
 
 # (nx, ny, levels, boundaries): sizes around a tile's edge, odd factors, flat and tall boxes
 GRIDS = [(96, 48, 5, "box"), (40, 136, 4, "plate"), (24, 200, 4, "pbc"), (72, 88, 4, "pbc_nmn"), (132, 20, 3, "nmn"),
-         (36, 12, 3, "pbc"), (128, 128, 7, "plate"), (33, 47, 1, "box"), (260, 196, 3, "pbc_plate")]
+         (36, 12, 3, "pbc"), (128, 128, 7, "plate"), (33, 47, 1, "box"), (260, 196, 3, "pbc_plate"),
+         # an odd number of columns over an even number of rows on a level that one CTA holds
+         (96, 64, 6, "box"), (33, 20, 1, "box"), (48, 64, 5, "pbc")]
 
 
 @pytest.mark.parametrize("small", [0, 300, 2000])
