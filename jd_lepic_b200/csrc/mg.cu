@@ -340,8 +340,10 @@ __device__ __forceinline__ void restriction(const Patch &g, int pbc, int ro, Mas
     const int lg = lanes_of(ic1 - ic0), lpr = 1 << lg;
     const int lane = threadIdx.x & (lpr - 1), sub = threadIdx.x >> lg, nsub = MGT >> lg;
     const int lny = g.wrap == 3 ? ny : ny - g.a0;    // local row of ny (periodic)
-    // r_pbc(x) of mg.f90:298-311 (zero where the reference leaves it unset)
+    // r_pbc(x) of mg.f90:298-311 (zero where the reference leaves it unset, and one past its end,
+    // which a free node of the right column asks for)
     auto rpbc = [&](int x) {
+        if (x > nx + 1) return 0.0;
         const int t = (lny + 1) * RP + x - g.ri0;
         bool set;
         if (x & 1) set = g.m(t) <= 0;

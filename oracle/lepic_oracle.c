@@ -517,7 +517,8 @@ static void restriction_nt(int nx, int ny, double hx, double hy, double eps0, co
     const int W = nx + 3, nx2 = nx / 2, ny2 = ny / 2, W2 = nx2 + 3;
     double *r_pbc = NULL;
     if (flag_pbc == 1) { /* :298-311 */
-        r_pbc = (double *)calloc((size_t)nx + 2, sizeof(double)); /* r_pbc(1:nx+1) */
+        /* r_pbc(1:nx+1); a free node of the right column reads one past it, which counts as zero */
+        r_pbc = (double *)calloc((size_t)nx + 3, sizeof(double));
         for (int i = 1; i <= nx2 + 1; i++) {
             int ir = 2 * i - 1;
             if (bcnd[ir + (ny + 1) * W] <= 0) {

@@ -69,6 +69,34 @@ def test_paths_match_oracle(gpu_lib, grid, small):
         s.close()
 
 
+@pytest.mark.parametrize("small", [0, 300, 2000])
+@pytest.mark.parametrize("size", [(32, 24, 3), (64, 48, 4), (96, 72, 4)])
+def test_free_right_column_between_periodic_edges(gpu_lib, size, small):
+    """Free nodes in the right column of a periodic deck: the restriction of the bottom row asks for
+    a residual one node past the grid, which counts as zero on every path."""
+    from jd_lepic_b200.simulation import GpuSimulation
+    nx, ny, ng = size
+    case = _case(nx, ny, ng, "pbc")
+    case.bcnd[:, nx + 1:] = 0
+    case.phi0 = configs.potentials(case.bcnd, {1: 5.0})
+    s = GpuSimulation(case, tile=(8, 8), load=False, capacity=64)
+    try:
+        s.set_options(mg_small_nodes=small)
+        rng = np.random.default_rng(nx)
+        X, Y = np.meshgrid(np.arange(nx + 1) / nx, np.arange(ny + 1) / ny)
+        rhs = 1.6e-3 * np.sin(3 * np.pi * X) * np.cos(2 * np.pi * Y) + 2e-4 * rng.normal(size=X.shape)
+        a = np.ascontiguousarray(rhs)
+        s.check(s.lib.lepic_gpu_set_grid(s.ctx, capi.GRID_RHS, a.ctypes.data_as(C.POINTER(C.c_double))), "set_grid")
+        st = s.solve(eps=1e-9, mode=capi.POISSON_FP64_MG, phi=case.phi0.copy())
+        ref = case.phi0.copy()
+        rc, ost = O.solve(O.make_cfg(case, s.sp), ref, rhs, case.bcnd, ng, 1e-9)
+        assert rc == 0 and ost.k < 20
+        assert (st["cycles"], st["sweeps_fine"]) == (ost.k, ost.sweeps_fine)
+        assert np.abs(st["phi"] - ref).max() <= 1e-13 * np.abs(ref).max()
+    finally:
+        s.close()
+
+
 def test_quotient_of_extreme_values(gpu_lib):
     """The update divides by the fixed diagonal with a corrected reciprocal where the dividend is in
     range and with the general division elsewhere: sources from 1e-300 to 1e200 in one deck."""
