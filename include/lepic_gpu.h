@@ -312,7 +312,11 @@ int lepic_gpu_deposit_noalloc(const uint32_t *X, const uint32_t *Y, const float 
                               double *np_out, void *stream);
 
 /* Raw device pointers of one species' SoA arrays (for in-process tools and tests):
- * X, Y are uint32 fixed point in cell units with `shift` fractional bits, VX/VY/VZ float. */
+ * X, Y are uint32 fixed point in cell units with `shift` fractional bits, VX/VY/VZ float.
+ * A species has two sets of arrays and this call returns the one in use: it stays in use through
+ * put_particles, load_particles and single pushes, while a sort (lepic_gpu_part_sorting, or the
+ * one inside lepic_gpu_step with the push that follows it) may go over to the other one: ask
+ * again after it. */
 int lepic_gpu_particle_arrays(lepic_ctx *ctx, int32_t ptype, void **X, void **Y, void **VX,
                               void **VY, void **VZ, int64_t *n_slots, int32_t *shift);
 

@@ -182,51 +182,67 @@ __global__ void k_put(const double *in, long long n, long long dst, double sx, d
     }
 }
 
-__global__ void k_put_counts(DevCounters *cnt, int sp, long long n) {
-    cnt->n_slots[sp] = n;
-    cnt->n_alive[sp] = n;
-    cnt->n_sorted[sp] = 0;
-    cnt->n_items[sp] = 0;
+// the end of a put whose particles were all inside the box: the n slots into the species' own
+// arrays, and its counts
+struct PutArrays {
+    uint32_t *X, *Y;
+    float *VX, *VY, *VZ, *Z;
+};
+__global__ void k_put_commit(const int *bad, PutArrays from, PutArrays to, long long n, DevCounters *cnt, int sp) {
+    if (*bad) return;
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+        to.X[k] = from.X[k]; to.Y[k] = from.Y[k];
+        to.VX[k] = from.VX[k]; to.VY[k] = from.VY[k]; to.VZ[k] = from.VZ[k];
+        if (to.Z) to.Z[k] = from.Z[k];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        cnt->n_slots[sp] = n;
+        cnt->n_alive[sp] = n;
+        cnt->n_sorted[sp] = 0;
+        cnt->n_items[sp] = 0;
+    }
 }
 
-// Replaces a species' particles.  They go to the buffer that is not in use, which takes over when
-// all of them have been found inside the box: a refused call leaves the species as it was.
+// Replaces a species' particles.  They go to the buffer that is not in use and are copied to the one
+// in use when all of them have been found inside the box: a refused call leaves the species as
+// it was, and pointers to its arrays show the new particles (the copy is 40 B per particle at the
+// device's rate, a thousandth of the way across the bus).
 int particles_put(lepic_ctx *c, int sp, const double *vxp, long long n) {
     SpeciesBuf &B = c->sp[sp];
     if (n < 0 || n > B.cap) { c->last_err = "particle count exceeds capacity"; return LEPIC_ECAPACITY; }
     const lepic_config &g = c->cfg;
-    if (n > 0) {
-        IoStage *S = n >= IO_PINNED ? io_stage(c) : nullptr;
-        const double sx = (double)(1u << c->S) / g.dx, sy = (double)(1u << c->S) / g.dy;
-        const long long xl = (long long)g.nx << c->S, yl = (long long)g.ny << c->S;
-        const long long chunk = io_chunk(c, 0);
-        double *const d[2] = {(double *)c->keys, (double *)c->perm};
-        int *const bad = c->blocksums;                   // scratch of the sort's scan
-        const int o = 1 - B.cur;
-        LCUDA(cudaMemsetAsync(bad, 0, sizeof(int), c->stream));
-        int b = 0;
-        for (long long k = 0; k < n; k += chunk, b ^= 1) {
-            const long long m = std::min(chunk, n - k);
-            const double *src = vxp + 6 * k;
-            if (S) {
-                if (k >= 2 * chunk) LCUDA(cudaEventSynchronize(S->ev[b]));   // the buffer's last chunk has left it
-                host_copy(S->h[b], src, 48 * (size_t)m);
-                src = S->h[b];
-            }
-            LCUDA(cudaMemcpyAsync(d[b], src, 48 * (size_t)m, cudaMemcpyHostToDevice, c->stream));
-            if (S) LCUDA(cudaEventRecord(S->ev[b], c->stream));
-            k_put<<<(int)std::min<long long>(div_up(m, 256), c->num_sms * 8), 256, 0, c->stream>>>(
-                d[b], m, k, sx, sy, xl, yl, B.X[o], B.Y[o], B.VX[o], B.VY[o], B.VZ[o], B.Z[o], bad);
-            LCUDA(cudaGetLastError());
+    IoStage *S = n >= IO_PINNED ? io_stage(c) : nullptr;
+    const double sx = (double)(1u << c->S) / g.dx, sy = (double)(1u << c->S) / g.dy;
+    const long long xl = (long long)g.nx << c->S, yl = (long long)g.ny << c->S;
+    const long long chunk = io_chunk(c, 0);
+    double *const d[2] = {(double *)c->keys, (double *)c->perm};
+    int *const bad = c->blocksums;                   // scratch of the sort's scan
+    const int cur = B.cur, o = 1 - cur;
+    LCUDA(cudaMemsetAsync(bad, 0, sizeof(int), c->stream));
+    int b = 0;
+    for (long long k = 0; k < n; k += chunk, b ^= 1) {
+        const long long m = std::min(chunk, n - k);
+        const double *src = vxp + 6 * k;
+        if (S) {
+            if (k >= 2 * chunk) LCUDA(cudaEventSynchronize(S->ev[b]));   // the buffer's last chunk has left it
+            host_copy(S->h[b], src, 48 * (size_t)m);
+            src = S->h[b];
         }
-        int hbad = 0;
-        LCUDA(cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-        LCUDA(cudaStreamSynchronize(c->stream));
-        if (hbad) { c->last_err = "particle outside the box"; return LEPIC_EINVAL; }
-        B.cur = o;
+        LCUDA(cudaMemcpyAsync(d[b], src, 48 * (size_t)m, cudaMemcpyHostToDevice, c->stream));
+        if (S) LCUDA(cudaEventRecord(S->ev[b], c->stream));
+        k_put<<<(int)std::min<long long>(div_up(m, 256), c->num_sms * 8), 256, 0, c->stream>>>(
+            d[b], m, k, sx, sy, xl, yl, B.X[o], B.Y[o], B.VX[o], B.VY[o], B.VZ[o], B.Z[o], bad);
+        LCUDA(cudaGetLastError());
     }
-    k_put_counts<<<1, 1, 0, c->stream>>>(c->dcnt, sp, n);
+    const PutArrays from = {B.X[o], B.Y[o], B.VX[o], B.VY[o], B.VZ[o], B.Z[o]};
+    const PutArrays to = {B.X[cur], B.Y[cur], B.VX[cur], B.VY[cur], B.VZ[cur], B.Z[cur]};
+    k_put_commit<<<(int)std::min<long long>(div_up(n, 256) + 1, c->num_sms * 8), 256, 0, c->stream>>>(bad, from, to, n,
+                                                                                                  c->dcnt, sp);
     LCUDA(cudaGetLastError());
+    int hbad = 0;
+    LCUDA(cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    LCUDA(cudaStreamSynchronize(c->stream));
+    if (hbad) { c->last_err = "particle outside the box"; return LEPIC_EINVAL; }
     B.ordered = false;
     return LEPIC_OK;
 }

@@ -86,3 +86,39 @@ def test_refused_put_changes_nothing(gpu_lib, at, what, size):
         assert np.array_equal(s.get_particles(0), before)
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("n", [1, 5000, CHUNK + 1, 5 * CHUNK])
+def test_arrays_in_use_show_a_put(gpu_lib, n):
+    """Pointers taken before a put show the particles put, those of a refused one the old ones."""
+    import torch
+
+    class Dev:
+        def __init__(self, ptr, kind):
+            self.__cuda_array_interface__ = {"shape": (n,), "typestr": kind, "data": (ptr, False), "version": 2}
+
+    from jd_lepic_b200.simulation import GpuSimulation
+    case = configs.case0(ppc=1, nx=32, ny=32)
+    s = GpuSimulation(case, tile=(8, 8), load=False, capacity=n)
+    try:
+        s.put_particles(0, _particles(case, n, 3))
+        for sort in (False, True):
+            if sort:
+                s.sort(0)                             # goes over to the other arrays
+            ptr = [C.c_void_p() for _ in range(5)]
+            s.check(s.lib.lepic_gpu_particle_arrays(s.ctx, 0, *[C.byref(v) for v in ptr], None, None), "particle_arrays")
+            p = _particles(case, n, 4)
+            p[::5, 3] = np.nan
+            s.put_particles(0, p)
+            bad = _particles(case, n, 5)
+            bad[n - 1, 0] = -1.0
+            with pytest.raises(capi.LepicError):
+                s.put_particles(0, bad)
+            got = [torch.as_tensor(Dev(v.value, "<i4" if q < 2 else "<f4"), device="cuda").cpu().numpy()
+                   for q, v in enumerate(ptr)]
+            for k, h in ((0, case.dx), (1, case.dy)):
+                assert np.array_equal(got[k].view(np.uint32), np.floor(p[:, k] * (2.0 ** 24 / h) + 0.5).astype(np.uint32))
+            for k in range(3):
+                assert np.array_equal(got[2 + k], p[:, 3 + k].astype(np.float32), equal_nan=True)
+    finally:
+        s.close()
