@@ -174,7 +174,7 @@ static int create_impl(lepic_ctx *c, const lepic_config *cfg, const int32_t *bcn
         LALLOC(B.prod, B.prod_cap);
     }
     // keys and perm also stage particles between host and device (backup.cu)
-    maxcap = std::max(maxcap, (long long)IO_MIN_SCRATCH);
+    maxcap = io_scratch(maxcap);
     c->scratch_cap = maxcap;
     LALLOC(c->keys, maxcap); LALLOC(c->perm, maxcap);
     LALLOC(c->counts, c->nkeys + 1); LALLOC(c->offsets, c->nkeys + 1); LALLOC(c->cursor, c->nkeys + 1);

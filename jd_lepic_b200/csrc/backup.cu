@@ -17,6 +17,7 @@
 // the device and is written as 0.  Reading unpacks FP64 chunks into the fixed-point and FP32
 // arrays after the occupied slots, then deposits every species (restart_OMP).
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -24,6 +25,7 @@
 #include <new>
 #include <thread>
 #include <vector>
+#include <sys/mman.h>
 #include "lepic_internal.cuh"
 
 #define BK_BLOCK 1024                 // slots per counting block
@@ -98,27 +100,39 @@ __global__ void k_unpack(const double *in, long long n, long long dst, double sx
 // ---------------------------------------------------------------------------------------
 // Particles to and from the host's FP64 vxp(6, n): the records cross in chunks, converted to and
 // from the device's arrays on the device.  The device side of a chunk is the sort's scratch (keys
-// and perm, free between sorts), taken in turns.  From IO_PINNED particles on, the host side goes
-// through two pinned buffers, filled or emptied by a few threads (one thread's copy, and its page
-// faults on a new array, are slower than the bus) beside the transfer and conversion of the
-// other chunk; fewer cross straight from and to the caller's array, since pinning the buffers at a
-// context's first call costs about 10 ms, more than it then saves.  (Converted by one host thread
-// between plain copies, put + sort + deposit + get of 2 x 1.3 M particles took 66 ms; so 21 ms, most
-// of it the page faults of the fresh host arrays.)
-#define IO_CHUNK (1ll << 17)          // particles per chunk at most (a multiple of BK_BLOCK): 6.3 MB (2^16: 31 ms)
-#define IO_PINNED (1ll << 19)
+// and perm, free between sorts).
+//  * From IO_LANED particles on, up to IO_LANES host threads take chunks in turn, each through two
+//    pinned buffers of its own: one thread's copy, and its page faults on a new array, are slower
+//    than the bus.  Put / get of 1.3 M particles: 2.9 / 2.7 ms, 5.8 into a new array; straight
+//    from and to the caller's array 4.9 / 3.6 and 14.  A context's first such call pays for the
+//    pinned memory, about 1 ms per MB (6.3 MB; with 12.6 MB steady times were the same), which a
+//    smaller number of particles does not earn back: 2^19 cross in 1.6 / 1.8 ms without.
+//  * Fewer cross straight from and to the caller's array, in chunks of up to IO_CHUNK particles taken
+//    by keys and perm in turn, which hold that many even where the species are smaller (a full
+//    species of 20000 in chunks of a third of the scratch: put 0.19, get 0.61 ms; so 0.11, 0.14).
+//    The driver is slow to copy into pages that do not exist yet, so they are made before
+//    (20000 particles into a new array 1.0 -> 0.43 ms, 300000 7.5 -> 3.6).
+// (Converted by one host thread between plain copies, put + sort + deposit + get of 2 x 1.3 M
+// particles took 66 ms; so 18.7 ms, most of it the page faults of the new host arrays.)
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23        // Linux 5.14; older headers do not name it
+#endif
+#define IO_CHUNK (1ll << 17)          // particles per direct chunk at most (a multiple of BK_BLOCK): 6.3 MB
+#define IO_LANED (1ll << 20)
+#define IO_LANES 4
+#define IO_LANE_CHUNK (16ll * BK_BLOCK)   // particles per pinned buffer: 786 kB
 struct IoStage {
-    double *h[2] = {nullptr, nullptr};
-    cudaEvent_t ev[2] = {nullptr, nullptr};
+    double *h = nullptr;
+    cudaEvent_t ev[IO_LANES][2] = {};
 };
 
 void io_free(lepic_ctx *c) {
     IoStage *S = (IoStage *)c->io;
     if (!S) return;
-    for (int k = 0; k < 2; k++) {
-        if (S->h[k]) cudaFreeHost(S->h[k]);
-        if (S->ev[k]) cudaEventDestroy(S->ev[k]);
-    }
+    if (S->h) cudaFreeHost(S->h);
+    for (auto &e : S->ev)
+        for (auto &v : e)
+            if (v) cudaEventDestroy(v);
     delete S;
     c->io = nullptr;
 }
@@ -130,41 +144,70 @@ static IoStage *io_stage(lepic_ctx *c) {
     IoStage *S = new (std::nothrow) IoStage;
     if (!S) return nullptr;
     c->io = S;
-    for (int k = 0; k < 2; k++)
-        if (cudaMallocHost((void **)&S->h[k], 48 * IO_CHUNK) != cudaSuccess ||
-            cudaEventCreateWithFlags(&S->ev[k], cudaEventDisableTiming) != cudaSuccess) {
-            cudaGetLastError();
-            io_free(c);
-            return nullptr;
-        }
-    return S;
+    bool ok = cudaMallocHost((void **)&S->h, 48 * IO_LANE_CHUNK * 2 * IO_LANES) == cudaSuccess;
+    for (auto &e : S->ev)
+        for (auto &v : e) ok = ok && cudaEventCreateWithFlags(&v, cudaEventDisableTiming) == cudaSuccess;
+    if (ok) return S;
+    cudaGetLastError();
+    io_free(c);
+    return nullptr;
 }
 
-// particles per chunk, a multiple of BK_BLOCK, behind `used` bytes of the scratch (which holds at
-// least one such block: IO_MIN_SCRATCH)
+// A get's block offsets and counts lie at the start of keys: bytes for nb blocks
+static long long io_offsets(long long nb) { return (8 * (nb + 1) + 4 * nb + 255) / 256 * 256; }
+
+// ints that keys and perm need to stage a species of `cap` slots
+long long io_scratch(long long cap) {
+    const long long nb = div_up(cap, BK_BLOCK);
+    return std::max(cap, (48 * std::min(IO_CHUNK, nb * BK_BLOCK) + io_offsets(nb)) / 4);
+}
+
+// particles per direct chunk, a multiple of BK_BLOCK, behind `used` bytes of the scratch
 static long long io_chunk(const lepic_ctx *c, long long used) {
-    const long long per = (4 * c->scratch_cap - used) / 48 / BK_BLOCK * BK_BLOCK;
-    return std::min(IO_CHUNK, per);
+    return std::min(IO_CHUNK, (4 * c->scratch_cap - used) / 48 / BK_BLOCK * BK_BLOCK);
 }
 
-// memcpy by up to four threads
-static void host_copy(void *dst, const void *src, size_t bytes) {
-    const size_t kPart = 1 << 20;
-    const int nt = (int)std::min<size_t>(std::min(4u, std::max(1u, std::thread::hardware_concurrency())), bytes / kPart);
-    if (nt < 2) { std::memcpy(dst, src, bytes); return; }
-    const size_t part = (bytes / nt + 4095) / 4096 * 4096;
-    std::vector<std::thread> pool;
-    size_t o = part;
+// A call's chunks, dispensed to a few host threads (this one among them; only this one when no
+// more can be started).  lane(t, next) works on as lane t, taking chunk numbers from next until
+// they run out, and returns the first error it meets.
+template <class Lane>
+static cudaError_t io_run(lepic_ctx *c, Lane lane) {
+    std::atomic<long long> next(0);
+    cudaError_t err[IO_LANES] = {};
+    std::thread pool[IO_LANES];
+    const int nt = (int)std::min((unsigned)IO_LANES, std::max(1u, std::thread::hardware_concurrency()));
     try {
-        for (int t = 1; t < nt && o < bytes; t++) {
-            const size_t k = std::min(part, bytes - o);
-            pool.emplace_back([=] { std::memcpy((char *)dst + o, (const char *)src + o, k); });
-            o += k;
+        for (int t = 1; t < nt; t++)
+            pool[t] = std::thread([&, t] {
+                err[t] = cudaSetDevice(c->dev);
+                if (err[t] == cudaSuccess) err[t] = lane(t, next);
+            });
+    } catch (...) { }                 // no more threads: those that run take all chunks
+    err[0] = lane(0, next);
+    for (auto &t : pool)
+        if (t.joinable()) t.join();
+    for (cudaError_t e : err)
+        if (e != cudaSuccess) {
+            cudaStreamSynchronize(c->stream);      // nothing of the call is left in flight
+            return e;
         }
-    } catch (...) { }                 // no more threads: this one copies what is left
-    std::memcpy(dst, src, std::min(part, bytes));
-    if (o < bytes) std::memcpy((char *)dst + o, (const char *)src + o, bytes - o);
-    for (auto &t : pool) t.join();
+    return cudaSuccess;
+}
+
+// makes the pages of an output that is about to be written (the contents stay), a few threads
+// together when it is large
+static void io_touch(lepic_ctx *c, double *out, size_t bytes) {
+    const uintptr_t kPage = 4096, kPart = 1 << 20;
+    const uintptr_t o = (uintptr_t)out / kPage * kPage, end = (uintptr_t)out + bytes;
+    auto touch = [](uintptr_t p, uintptr_t e) {
+        if (p >= e || madvise((void *)p, e - p, MADV_POPULATE_WRITE) == 0) return;
+        for (; p < e; p += kPage) __atomic_fetch_add((char *)p, 0, __ATOMIC_RELAXED);   // a system that does not have it
+    };
+    if (bytes < 4 * kPart) { touch(o, end); return; }
+    io_run(c, [&](int, std::atomic<long long> &next) {
+        for (uintptr_t p; (p = o + kPart * (uintptr_t)next++) < end;) touch(p, std::min(end, p + kPart));
+        return cudaSuccess;
+    });
 }
 
 // n host particles into slots dst ..; one outside the box (or at no number) sets *bad
@@ -211,28 +254,44 @@ int particles_put(lepic_ctx *c, int sp, const double *vxp, long long n) {
     SpeciesBuf &B = c->sp[sp];
     if (n < 0 || n > B.cap) { c->last_err = "particle count exceeds capacity"; return LEPIC_ECAPACITY; }
     const lepic_config &g = c->cfg;
-    IoStage *S = n >= IO_PINNED ? io_stage(c) : nullptr;
+    IoStage *S = n >= IO_LANED ? io_stage(c) : nullptr;
     const double sx = (double)(1u << c->S) / g.dx, sy = (double)(1u << c->S) / g.dy;
     const long long xl = (long long)g.nx << c->S, yl = (long long)g.ny << c->S;
-    const long long chunk = io_chunk(c, 0);
     double *const d[2] = {(double *)c->keys, (double *)c->perm};
     int *const bad = c->blocksums;                   // scratch of the sort's scan
     const int cur = B.cur, o = 1 - cur;
     LCUDA(cudaMemsetAsync(bad, 0, sizeof(int), c->stream));
-    int b = 0;
-    for (long long k = 0; k < n; k += chunk, b ^= 1) {
-        const long long m = std::min(chunk, n - k);
-        const double *src = vxp + 6 * k;
-        if (S) {
-            if (k >= 2 * chunk) LCUDA(cudaEventSynchronize(S->ev[b]));   // the buffer's last chunk has left it
-            host_copy(S->h[b], src, 48 * (size_t)m);
-            src = S->h[b];
-        }
-        LCUDA(cudaMemcpyAsync(d[b], src, 48 * (size_t)m, cudaMemcpyHostToDevice, c->stream));
-        if (S) LCUDA(cudaEventRecord(S->ev[b], c->stream));
+    auto convert = [&](const double *in, long long k, long long m) {
         k_put<<<(int)std::min<long long>(div_up(m, 256), c->num_sms * 8), 256, 0, c->stream>>>(
-            d[b], m, k, sx, sy, xl, yl, B.X[o], B.Y[o], B.VX[o], B.VY[o], B.VZ[o], B.Z[o], bad);
-        LCUDA(cudaGetLastError());
+            in, m, k, sx, sy, xl, yl, B.X[o], B.Y[o], B.VX[o], B.VY[o], B.VZ[o], B.Z[o], bad);
+        return cudaGetLastError();
+    };
+    if (S) {
+        const cudaError_t er = io_run(c, [&](int t, std::atomic<long long> &next) {
+            cudaError_t e = cudaSuccess;
+            for (int i = 0; e == cudaSuccess; i++) {
+                const long long k = IO_LANE_CHUNK * next++, m = std::min(IO_LANE_CHUNK, n - k);
+                if (m <= 0) break;
+                const int b = i & 1;
+                double *const h = S->h + 6 * IO_LANE_CHUNK * (2 * t + b), *const q = d[b] + 6 * IO_LANE_CHUNK * t;
+                if (i >= 2) e = cudaEventSynchronize(S->ev[t][b]);   // the buffer's last chunk has left it
+                if (e != cudaSuccess) break;
+                std::memcpy(h, vxp + 6 * k, 48 * (size_t)m);
+                e = cudaMemcpyAsync(q, h, 48 * (size_t)m, cudaMemcpyHostToDevice, c->stream);
+                if (e == cudaSuccess) e = cudaEventRecord(S->ev[t][b], c->stream);
+                if (e == cudaSuccess) e = convert(q, k, m);
+            }
+            return e;
+        });
+        LCUDA(er);
+    } else {
+        const long long chunk = io_chunk(c, 0);
+        int b = 0;
+        for (long long k = 0; k < n; k += chunk, b ^= 1) {
+            const long long m = std::min(chunk, n - k);
+            LCUDA(cudaMemcpyAsync(d[b], vxp + 6 * k, 48 * (size_t)m, cudaMemcpyHostToDevice, c->stream));
+            LCUDA(convert(d[b], k, m));
+        }
     }
     const PutArrays from = {B.X[o], B.Y[o], B.VX[o], B.VY[o], B.VZ[o], B.Z[o]};
     const PutArrays to = {B.X[cur], B.Y[cur], B.VX[cur], B.VY[cur], B.VZ[cur], B.Z[cur]};
@@ -256,8 +315,8 @@ int particles_get(lepic_ctx *c, int sp, double *vxp, long long cap, long long *n
     const long long ns = c->hcnt->n_slots[sp], nb = div_up(ns, BK_BLOCK);
     if (n_out) *n_out = 0;
     if (ns == 0) return LEPIC_OK;
-    // the scratch: block offsets and counts at the start of keys, then one chunk; perm the other
-    const long long used = (8 * (nb + 1) + 4 * nb + 255) / 256 * 256;
+    // the scratch: block offsets and counts at the start of keys, chunks behind them and in perm
+    const long long used = io_offsets(nb);
     long long *const d_off = (long long *)c->keys;
     int *const d_cnt = (int *)(d_off + nb + 1);
     double *const d[2] = {(double *)((char *)c->keys + used), (double *)c->perm};
@@ -271,32 +330,53 @@ int particles_get(lepic_ctx *c, int sp, double *vxp, long long cap, long long *n
     const long long total = off[nb];
     if (n_out) *n_out = total;
     if (vxp) {
-        IoStage *S = total >= IO_PINNED ? io_stage(c) : nullptr;
+        IoStage *S = total >= IO_LANED ? io_stage(c) : nullptr;
         LCUDA(cudaMemcpyAsync(d_off, off.data(), sizeof(long long) * (nb + 1), cudaMemcpyHostToDevice, c->stream));
         const double ux = g.dx * std::ldexp(1.0, -c->S), uy = g.dy * std::ldexp(1.0, -c->S);
-        const long long per = io_chunk(c, used) / BK_BLOCK;
-        long long at[2] = {0, 0}, len[2] = {0, 0};   // where a buffer's particles go, and how many
-        auto finish = [&](int b) {
-            const cudaError_t e = cudaEventSynchronize(S->ev[b]);
-            if (e == cudaSuccess) host_copy(vxp + 6 * at[b], S->h[b], 48 * (size_t)len[b]);
-            return e;
-        };
-        int b = 0, pending = 0;
-        for (long long b0 = 0; b0 < nb && off[b0] < cap; b0 += per, b ^= 1) {
-            const long long bn = std::min(per, nb - b0);
+        // blocks b0 .. b0 + bn packed into q and copied to h; how many particles, up to cap
+        auto fetch = [&](long long b0, long long bn, double *q, double *h, long long &len) {
             k_pack<<<(unsigned)bn, BK_BLOCK, 0, c->stream>>>(B.X[B.cur], B.Y[B.cur], B.VX[B.cur], B.VY[B.cur], B.VZ[B.cur],
-                                                             B.Z[B.cur], ns, b0, d_off, ux, uy, d[b]);
-            LCUDA(cudaGetLastError());
-            at[b] = off[b0];
-            len[b] = std::min(off[b0 + bn], cap) - off[b0];
-            LCUDA(cudaMemcpyAsync(S ? S->h[b] : vxp + 6 * at[b], d[b], 48 * (size_t)len[b], cudaMemcpyDeviceToHost, c->stream));
-            if (!S) continue;
-            LCUDA(cudaEventRecord(S->ev[b], c->stream));
-            if (pending) LCUDA(finish(b ^ 1));       // the chunk before, while this one is on its way
-            pending = 1;
+                                                             B.Z[B.cur], ns, b0, d_off, ux, uy, q);
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) return e;
+            len = std::min(off[b0 + bn], cap) - off[b0];
+            return cudaMemcpyAsync(h, q, 48 * (size_t)len, cudaMemcpyDeviceToHost, c->stream);
+        };
+        if (S) {
+            const cudaError_t er = io_run(c, [&](int t, std::atomic<long long> &next) {
+                const long long per = IO_LANE_CHUNK / BK_BLOCK;
+                long long at[2] = {0, 0}, len[2] = {0, 0};   // where a buffer's particles go, and how many
+                auto buf = [&](int b) { return S->h + 6 * IO_LANE_CHUNK * (2 * t + b); };
+                auto finish = [&](int b) {
+                    if (!len[b]) return cudaSuccess;
+                    const cudaError_t e = cudaEventSynchronize(S->ev[t][b]);
+                    if (e == cudaSuccess) std::memcpy(vxp + 6 * at[b], buf(b), 48 * (size_t)len[b]);
+                    len[b] = 0;
+                    return e;
+                };
+                cudaError_t e = cudaSuccess;
+                int b = 0;
+                for (; e == cudaSuccess; b ^= 1) {
+                    const long long b0 = per * next++;
+                    if (b0 >= nb || off[b0] >= cap) break;
+                    at[b] = off[b0];
+                    e = fetch(b0, std::min(per, nb - b0), d[b] + 6 * IO_LANE_CHUNK * t, buf(b), len[b]);
+                    if (e == cudaSuccess) e = cudaEventRecord(S->ev[t][b], c->stream);
+                    if (e == cudaSuccess) e = finish(b ^ 1);   // the chunk before, while this one is on its way
+                }
+                return e == cudaSuccess ? finish(b ^ 1) : e;
+            });
+            LCUDA(er);
+        } else {
+            io_touch(c, vxp, 48 * (size_t)std::min(total, std::max(cap, 0ll)));
+            const long long per = io_chunk(c, used) / BK_BLOCK;
+            int b = 0;
+            for (long long b0 = 0; b0 < nb && off[b0] < cap; b0 += per, b ^= 1) {
+                long long len = 0;
+                LCUDA(fetch(b0, std::min(per, nb - b0), d[b], vxp + 6 * off[b0], len));
+            }
+            LCUDA(cudaStreamSynchronize(c->stream));
         }
-        if (pending) LCUDA(finish(b ^ 1));
-        else LCUDA(cudaStreamSynchronize(c->stream));
     }
     if (vxp && total > cap) { c->last_err = "output capacity too small"; return LEPIC_ECAPACITY; }
     return LEPIC_OK;

@@ -455,7 +455,7 @@ bool push_needs_general(const lepic_ctx *c, int s);
 int particles_load(lepic_ctx *c, const lepic_load_spec *spec);
 int particles_put(lepic_ctx *c, int ptype, const double *vxp, long long n);
 void io_free(lepic_ctx *c);
-#define IO_MIN_SCRATCH 16384   // ints: a block of 1024 particles at 48 B, and its offsets
+long long io_scratch(long long cap);
 int particles_get(lepic_ctx *c, int ptype, double *vxp, long long cap, long long *n_out);
 int sources_before_push(lepic_ctx *c, int it);
 int sources_after_push(lepic_ctx *c, int it);

@@ -10,7 +10,7 @@ from jd_lepic_b200 import _capi as capi, configs
 
 pytestmark = pytest.mark.gpu
 
-CHUNK = 131072     # the largest chunk; pinned buffers from 4 of them on
+CHUNK = 131072     # the largest chunk; several host threads and pinned buffers from 8 of them on
 
 
 def _particles(case, n, seed):
@@ -32,7 +32,8 @@ def _stored(p, case):
     return q
 
 
-@pytest.mark.parametrize("n", [0, 1, 1023, CHUNK - 1, CHUNK, CHUNK + 1, 2 * CHUNK + 5, 5 * CHUNK - 700, 6 * CHUNK + 3])
+@pytest.mark.parametrize("n", [0, 1, 1023, CHUNK - 1, CHUNK, CHUNK + 1, 2 * CHUNK + 5, 5 * CHUNK - 700,
+                               8 * CHUNK - 1, 8 * CHUNK, 13 * CHUNK + 700])
 def test_round_trip(gpu_lib, n):
     from jd_lepic_b200.simulation import GpuSimulation
     case = configs.case0(ppc=1, nx=64, ny=48)
@@ -63,7 +64,7 @@ def test_round_trip(gpu_lib, n):
         s.close()
 
 
-@pytest.mark.parametrize("size", [2, 4])
+@pytest.mark.parametrize("size", [2, 8])
 @pytest.mark.parametrize("at", [0, CHUNK - 1, 2 * CHUNK + 3])
 @pytest.mark.parametrize("what", [(0, -1e-4), (1, 1.0), (0, np.nan), (1, np.inf)])
 def test_refused_put_changes_nothing(gpu_lib, at, what, size):
@@ -88,7 +89,7 @@ def test_refused_put_changes_nothing(gpu_lib, at, what, size):
         s.close()
 
 
-@pytest.mark.parametrize("n", [1, 5000, CHUNK + 1, 5 * CHUNK])
+@pytest.mark.parametrize("n", [1, 5000, CHUNK + 1, 8 * CHUNK])
 def test_arrays_in_use_show_a_put(gpu_lib, n):
     """Pointers taken before a put show the particles put, those of a refused one the old ones."""
     import torch
@@ -120,5 +121,25 @@ def test_arrays_in_use_show_a_put(gpu_lib, n):
                 assert np.array_equal(got[k].view(np.uint32), np.floor(p[:, k] * (2.0 ** 24 / h) + 0.5).astype(np.uint32))
             for k in range(3):
                 assert np.array_equal(got[2 + k], p[:, 3 + k].astype(np.float32), equal_nan=True)
+    finally:
+        s.close()
+
+
+@pytest.mark.parametrize("capacity", [1024, 20000, CHUNK, 700000])
+def test_full_species_crosses_in_large_chunks(gpu_lib, capacity):
+    """A species as large as the sort's scratch allows, put, sorted and read back: the scratch holds a
+    chunk of up to 131072 particles beside the read's block offsets."""
+    from jd_lepic_b200.simulation import GpuSimulation
+    case = configs.case0(ppc=1, nx=48, ny=40)
+    case.ng = 1
+    s = GpuSimulation(case, tile=(8, 8), load=False, capacity=capacity)
+    try:
+        p = _particles(case, capacity, 9)
+        s.put_particles(0, p)
+        s.put_particles(1, p[::-1])
+        s.sort(0)
+        assert np.array_equal(s.get_particles(1), _stored(p[::-1], case))
+        a, b = s.get_particles(0), _stored(p, case)
+        assert np.array_equal(a[np.lexsort(a.T)], b[np.lexsort(b.T)])
     finally:
         s.close()
