@@ -34,15 +34,22 @@ __global__ void k_na_zero(unsigned long long *acc, long long nn) {
         acc[t] = 0ull;
 }
 
-// Each thread walks `per` consecutive slots and keeps a run of particles in one cell as its
-// moments (count, sum fx, sum fy, sum fx fy), which give the sum of the particles' rounded weights
-// exactly, so that one run costs four atomics instead of four per particle.  Without rounding
-// (sh <= 0) the products are only shifted up.  With it each weight is (v + h) >> sh, h = 2^(sh-1),
-// and a run's sum is (sum v + n h - sum of the bits cut off) >> sh: the cell size 2^S being a
-// multiple of 2^sh, the four products are +-fx fy modulo 2^sh, so r = (fx fy + h) mod 2^sh gives
-// the bits cut off for two of the nodes and 2^sh - r (0 for r = 0) for the other two.
+// A warp takes 32 Q consecutive slots at a time, Q per lane, and keeps a run of particles in one
+// cell as its moments (count, sum fx, sum fy, sum fx fy), which give the sum of the particles'
+// rounded weights exactly, so that one run costs four atomics instead of four per particle: each
+// lane's own runs first, then its last one joined with the neighbours' where they are in the same
+// cell.  Sorted arrays come in long runs; arrays in random order come in runs of one, skip the
+// joining and are bound by their atomics.  Every load of a warp covers whole lines whatever the
+// arrays' alignment.  1e7 particles on 511 x 300: in cell order 353 us with four atomics per
+// particle, 58 so (2 TB/s of their 12 B); in random order 232 and 222.  (A thread that walked 32
+// slots of its own read lines 128 bytes apart: 71 us in order, 259 in random order, 138 and 306
+// where the arrays are not 16-byte aligned.)
+// Without rounding (sh <= 0) the products are only shifted up.  With it each weight is (v + h) >> sh,
+// h = 2^(sh-1), and a run's sum is (sum v + n h - sum of the bits cut off) >> sh: the cell size 2^S
+// being a multiple of 2^sh, the four products are +-fx fy modulo 2^sh, so r = (fx fy + h) mod 2^sh
+// gives the bits cut off for two of the nodes and 2^sh - r (0 for r = 0) for the other two.
 struct NaRun {
-    int cx, cy;                 // its cell; cx < 0: none
+    int node;                   // its cell's first node; < 0: none
     uint32_t n, sx, sy;         // n: count (bits 0..7), nonzero remainders (8..15), their sum (16..)
     uint64_t sxy;
 };
@@ -59,69 +66,74 @@ __device__ __forceinline__ void na_add(const NaRun &r, int S, int sh, int W, uns
         w0 <<= -sh; w1 <<= -sh; w2 <<= -sh; w3 <<= -sh;
     }
     // cx <= nx-1 and cy <= ny-1, so the four nodes (cx+1..cx+2, cy+1..cy+2) are inside
-    unsigned long long *q = acc + ((long long)r.cx + 1) + ((long long)r.cy + 1) * W;
+    unsigned long long *q = acc + r.node;
     if (w0) atomicAdd(q, (unsigned long long)w0);
     if (w1) atomicAdd(q + 1, (unsigned long long)w1);
     if (w2) atomicAdd(q + W + 1, (unsigned long long)w2);
     if (w3) atomicAdd(q + W, (unsigned long long)w3);
 }
 
-#define NA_PER_MAX 32   // slots per thread at most (the run's packed counts hold up to 255)
+// A run of 128 slots at most fits: its packed counts hold up to 255, its sums of offsets below
+// 2^24 stay below 2^31.  Up to NA_SMALL slots a lane takes one of them: with four too few warps are in
+// flight (2e5 in random order on 511 x 300: 21.5 us against 19.5, as many in order 17.4 both);
+// beyond it the longer runs pay (1e6 in order 23.5 us with one, 21.4 with four).
+#define NA_SMALL (1ll << 19)
 
-// VEC: X, Y and VX are 16-byte aligned, four slots per load; else one slot at a time.  `per` is a
-// multiple of 4.
-template <bool VEC>
+// Q: slots per lane (1 or 4)
+template <int Q>
 __global__ void __launch_bounds__(256) k_na_deposit(const uint32_t *X, const uint32_t *Y, const float *VX, long long n,
-                                                    int per, int S, int nx, int ny, unsigned long long *acc) {
+                                                    int S, int nx, int ny, unsigned long long *acc) {
+    const unsigned full = 0xffffffffu;
     const uint32_t mask = (1u << S) - 1u;
     const int sh = 2 * S - LEPIC_DEP_SHIFT;
     const uint32_t rh = sh > 0 ? 1u << (sh - 1) : 0u, rm = sh > 0 ? (1u << sh) - 1u : 0u;
-    const int W = nx + 3;
-    for (long long i0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * per; i0 < n;
-         i0 += (long long)gridDim.x * blockDim.x * per) {
+    const int W = nx + 3, lane = threadIdx.x & 31;
+    const long long w0 = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
+    for (long long base = w0 * (32 * Q); base < n; base += nw * (32 * Q)) {   // the same for a whole warp
+        const long long i = base + Q * lane;
+        uint32_t xs[Q], ys[Q];
+        float vs[Q];
+#pragma unroll
+        for (int p = 0; p < Q; p++) {
+            const bool in = i + p < n;
+            xs[p] = in ? X[i + p] : 0u;
+            ys[p] = in ? Y[i + p] : 0u;
+            vs[p] = !in ? __int_as_float(HOLE_NAN) : (VX ? VX[i + p] : 0.0f);
+        }
         NaRun r;
-        r.cx = -1; r.cy = 0; r.n = r.sx = r.sy = 0u; r.sxy = 0ull;
-        const long long i1 = min(i0 + per, n);
-        for (long long i = i0; i < i1; i += 4) {
-            uint32_t xs[4], ys[4];
-            float vs[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if (VEC && i + 4 <= n) {
-                const uint4 x = *reinterpret_cast<const uint4 *>(X + i), y = *reinterpret_cast<const uint4 *>(Y + i);
-                xs[0] = x.x; xs[1] = x.y; xs[2] = x.z; xs[3] = x.w;
-                ys[0] = y.x; ys[1] = y.y; ys[2] = y.z; ys[3] = y.w;
-                if (VX) {
-                    const float4 v = *reinterpret_cast<const float4 *>(VX + i);
-                    vs[0] = v.x; vs[1] = v.y; vs[2] = v.z; vs[3] = v.w;
-                }
+        r.node = -1; r.n = r.sx = r.sy = 0u; r.sxy = 0ull;
+#pragma unroll
+        for (int p = 0; p < Q; p++) {
+            if (isnan(vs[p])) continue; // a hole left by a lost particle, or past the end
+            const uint32_t cx = xs[p] >> S, cy = ys[p] >> S;
+            if (cx >= (uint32_t)nx || cy >= (uint32_t)ny) continue; // outside the box: not deposited
+            const uint32_t fx = xs[p] & mask, fy = ys[p] & mask;
+            const uint64_t fxy = (uint64_t)fx * fy;
+            const uint32_t rem = ((uint32_t)fxy + rh) & rm;
+            const uint32_t one = (rem << 16) + (rem ? 257u : 1u);
+            const int node = (int)cx + 1 + ((int)cy + 1) * W;
+            if (node != r.node) {
+                if (r.node >= 0) na_add(r, S, sh, W, acc);
+                r.node = node;
+                r.n = one; r.sx = fx; r.sy = fy; r.sxy = fxy;
             } else {
-#pragma unroll
-                for (int p = 0; p < 4; p++) {
-                    const bool in = i + p < n;
-                    xs[p] = in ? X[i + p] : 0u;
-                    ys[p] = in ? Y[i + p] : 0u;
-                    if (!in) vs[p] = __int_as_float(HOLE_NAN);
-                    else if (VX) vs[p] = VX[i + p];
-                }
-            }
-#pragma unroll
-            for (int p = 0; p < 4; p++) {
-                if (isnan(vs[p])) continue; // a hole left by a lost particle, or past the end
-                const uint32_t cx = xs[p] >> S, cy = ys[p] >> S;
-                if (cx >= (uint32_t)nx || cy >= (uint32_t)ny) continue; // outside the box: not deposited
-                const uint32_t fx = xs[p] & mask, fy = ys[p] & mask;
-                const uint64_t fxy = (uint64_t)fx * fy;
-                const uint32_t rem = ((uint32_t)fxy + rh) & rm;
-                const uint32_t one = (rem << 16) + (rem ? 257u : 1u);
-                if ((int)cx != r.cx || (int)cy != r.cy) {
-                    if (r.cx >= 0) na_add(r, S, sh, W, acc);
-                    r.cx = (int)cx; r.cy = (int)cy;
-                    r.n = one; r.sx = fx; r.sy = fy; r.sxy = fxy;
-                } else {
-                    r.n += one; r.sx += fx; r.sy += fy; r.sxy += fxy;
-                }
+                r.n += one; r.sx += fx; r.sy += fy; r.sxy += fxy;
             }
         }
-        if (r.cx >= 0) na_add(r, S, sh, W, acc);
+        // the lanes' last runs: a segment is a run of lanes in one cell, summed into its last lane
+        const int before = __shfl_up_sync(full, r.node, 1);
+        const unsigned heads = __ballot_sync(full, lane == 0 || before != r.node);
+        const int start = 31 - __clz(heads & (full >> (31 - lane)));
+        for (int o = 1; o < 32; o <<= 1) {
+            const bool take = lane - o >= start;
+            if (!__any_sync(full, take)) break;      // no segment is longer than o lanes
+            const uint32_t n2 = __shfl_up_sync(full, r.n, o), x2 = __shfl_up_sync(full, r.sx, o), y2 = __shfl_up_sync(full, r.sy, o);
+            const uint64_t xy2 = __shfl_up_sync(full, r.sxy, o);
+            if (take) { r.n += n2; r.sx += x2; r.sy += y2; r.sxy += xy2; }
+        }
+        const bool last = lane == 31 || ((heads >> (lane + 1)) & 1u);
+        if (r.node >= 0 && last) na_add(r, S, sh, W, acc);
     }
 }
 
@@ -165,15 +177,10 @@ extern "C" int lepic_gpu_deposit_noalloc(const uint32_t *X, const uint32_t *Y, c
     const int grid = 4 * sms;
     k_na_zero<<<grid, 256, 0, st>>>(acc, nn); // the array keeps the previous call's sums
     if (n > 0) {
-        // slots per thread: as many as still fill the GPU with threads, so that sorted arrays come
-        // in long runs (1e7 sorted particles on 511 x 300: 362 us
-        // with four atomics per particle, 59 us so, 2 TB/s of the 12 B per particle)
-        const long long threads = (long long)sms * 2048;
-        const int per = (int)std::min<long long>(NA_PER_MAX, std::max<long long>(4, (n / threads + 3) / 4 * 4));
-        const int blocks = (int)std::min<long long>(16ll * sms, (n + 256ll * per - 1) / (256ll * per));
-        const bool vec = (((uintptr_t)X | (uintptr_t)Y | (uintptr_t)VX) & 15) == 0;
-        if (vec) k_na_deposit<true><<<blocks, 256, 0, st>>>(X, Y, VX, n, per, shift, nx, ny, acc);
-        else k_na_deposit<false><<<blocks, 256, 0, st>>>(X, Y, VX, n, per, shift, nx, ny, acc);
+        const int q = n <= NA_SMALL ? 1 : 4;
+        const int blocks = (int)std::min<long long>(16ll * sms, (n + 256 * q - 1) / (256 * q));
+        if (q == 1) k_na_deposit<1><<<blocks, 256, 0, st>>>(X, Y, VX, n, shift, nx, ny, acc);
+        else k_na_deposit<4><<<blocks, 256, 0, st>>>(X, Y, VX, n, shift, nx, ny, acc);
     }
     k_na_finish<<<grid, 256, 0, st>>>(acc, kq, k1, nn, np_out);
     return cudaGetLastError() == cudaSuccess ? LEPIC_OK : LEPIC_ECUDA;

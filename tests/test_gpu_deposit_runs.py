@@ -53,7 +53,11 @@ def test_noalloc_is_exact(gpu_lib, size, order):
     nn = (nx + 3) * (ny + 3)
     rng = np.random.default_rng(ny)
     kq = torch.from_numpy(rng.integers(1, 3, nn).astype(np.float64)).cuda()
-    for n, lead in ((1, 0), (5, 1), (1023, 3), (200003, 0), (200003, 2), (3000017, 0)):
+    # the largest (where weights are rounded): several passes of the whole grid of warps, and in cell
+    # order every warp's 128 slots in one cell or two: the packed counts and remainder sums at their largest
+    large = ((20000003, 0), (20000003, 1)) if size in ((40, 56), (511, 33)) else ()
+    small = 1 << 19                           # one slot per lane up to here, four beyond
+    for n, lead in ((1, 0), (5, 1), (1023, 3), (200003, 0), (200003, 2), (small, 1), (small + 1, 3), (3000017, 0)) + large:
         X = rng.integers(0, nx << S, n, dtype=np.int64)
         Y = rng.integers(0, ny << S, n, dtype=np.int64)
         if order == "sorted":
