@@ -251,9 +251,11 @@ typedef struct lepic_options {
     int32_t mx_coarse_direct;    /* 1: the on-chip levels' top level (at most 2048 unknowns) solved
                                     exactly by its precomputed inverse, applied by every CTA
                                     (default); 0: CTA 0 cycles through the on-chip levels         */
-    int32_t mg_small_nodes;      /* FP64 V-cycle: levels of at most this many nodes on CTA 0 (4500;
-                                    at most 2000 are, larger ones being faster in tiles)           */
-    int32_t ctas_per_sm;         /* CTAs per SM of the cooperative solver kernels (3)                */
+    int32_t mg_small_nodes;      /* FP64 V-cycle: levels of at most this many nodes on CTA 0 (2000), as
+                                    far as its shared memory holds them (one level of up to about
+                                    4900 nodes and the coarser ones)                               */
+    int32_t ctas_per_sm;         /* CTAs per SM of the mixed-precision solver's cooperative kernel (3);
+                                    the FP64 multigrid's takes one SM per CTA                      */
     int32_t barrier_extra;       /* test hook, 0 in use: the solvers' grid barriers wait for this
                                     many CTAs beyond the launch, so the first wait runs out (after
                                     about 2 s), the kernel ends and the call returns LEPIC_ETIMEOUT */

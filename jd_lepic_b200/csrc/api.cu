@@ -308,7 +308,7 @@ static lepic_options default_options() {
     o.mx_tiled = 1;
     o.mx_max_iter = 200;
     o.mx_coarse_direct = 1;
-    o.mg_small_nodes = 4500;
+    o.mg_small_nodes = 2000;
     o.ctas_per_sm = 3;
     o.barrier_extra = 0;
     o.fortran_max_subrecord = 2147483639ll;
@@ -341,8 +341,6 @@ extern "C" int lepic_gpu_set_options(lepic_ctx *c, const lepic_options *in) {
     if (relaunch) {
         c->mg_grid_mixed = 0;  // sized again at the next mixed solve
         c->mg_grid_mixed64 = 0;
-        int r = mg_init(c);
-        if (r != LEPIC_OK) return r;
     }
     return LEPIC_OK;
 }

@@ -20,7 +20,7 @@
 //    number of sweeps the stage took in the previous cycle.  The decisions are taken afterwards
 //    from the K sums, which are the reference's: if it would have stopped earlier, the pass is
 //    run again from its untouched input with that many sweeps; if not yet, another pass follows.
-//  * Levels of at most small_nodes nodes live in CTA 0's shared memory (u, b, mask) for the
+//  * Levels of at most mg_small_nodes nodes live in CTA 0's shared memory (u, b, mask) for the
 //    whole solve, under the same prediction: K sweeps, then one reduction of their K sums.
 //  * A sweep in shared memory is bound by its loads and by what surrounds the arithmetic: u, b
 //    and the mask are kept by colour (unit stride, two wavefronts per load instead of four),
@@ -854,11 +854,12 @@ __global__ void __launch_bounds__(MGT, 1) k_mg_solve(const __grid_constant__ MGP
 }
 
 // ---------------------------------------------------------------------------------------
-// Where one CTA's sweep of a level, bound by its SM's shared-memory loads and FP64 units, costs as
-// much as a tile pass over the whole GPU with its grid barrier: 65^2 nodes take 11.4 / 35 us for a
-// stage of 2 / 10 sweeps on CTA 0 and 10 / 33 us in tiles (128^2 solve 0.69 against 0.64 ms), 49 x 33
-// nodes are 5 % of the 384 x 256 solve faster on CTA 0, 33^2 nodes 10 % of the 128^2 solve.
-#define MG_CTA0_NODES 2000
+// The levels of at most lepic_options::mg_small_nodes nodes are CTA 0's, as far as its shared memory
+// holds them (one level of up to about 4900 nodes and the coarser ones).  The default of 2000 is
+// where one CTA's sweep, bound by its SM's shared-memory loads and FP64 units, costs as much as a
+// tile pass over the whole GPU with its grid barrier: 65^2 nodes take 11.4 / 35 us for a stage of
+// 2 / 10 sweeps on CTA 0 and 10 / 33 us in tiles (128^2 solve 0.69 against 0.64 ms), 49 x 33 nodes
+// are 5 % of the 384 x 256 solve faster on CTA 0, 33^2 nodes 10 % of the 128^2 solve.
 #define MG_SMEM (224 * 1024)   // dynamic shared memory per CTA (one per SM)
 
 static MGP mg_params(lepic_ctx *c, double eps, int mode) {
@@ -877,9 +878,9 @@ static MGP mg_params(lepic_ctx *c, double eps, int mode) {
         d.u2 = l == 0 ? c->cg_ap : a.u2;
     }
     P.ng = c->nlev;
-    // the CTA-0 part: the coarsest levels, as long as each has at most small_nodes nodes (and at
-    // most MG_CTA0_NODES) and they fit in shared memory together
-    const long long small_nodes = std::min<long long>(c->opt.mg_small_nodes, MG_CTA0_NODES);
+    // the CTA-0 part: the coarsest levels, as long as each has at most mg_small_nodes nodes and they
+    // fit in shared memory together (a level's residual in the slots' space)
+    const long long small_nodes = c->opt.mg_small_nodes;
     const long long room = MG_SMEM / 8 - MG_SLOTS;      // doubles
     long long total = 0;                                // nodes of the CTA-0 part, both colours' padding included
     P.Ls = c->nlev;
@@ -933,7 +934,7 @@ int mg_init(lepic_ctx *c) {
     LCUDA(cudaFuncSetAttribute(k_mg_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM));
     LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mg_solve, MGT, MG_SMEM));
     if (occ < 1) { c->last_err = "multigrid kernel does not fit on an SM"; return LEPIC_ECUDA; }
-    c->mg_grid = c->num_sms * std::max(1, std::min(occ, (int)c->opt.ctas_per_sm));
+    c->mg_grid = c->num_sms;       // a CTA takes an SM's shared memory
     return LEPIC_OK;
 }
 

@@ -41,7 +41,7 @@ GRIDS = [(96, 48, 5, "box"), (40, 136, 4, "plate"), (24, 200, 4, "pbc"), (72, 88
          (96, 64, 6, "box"), (33, 20, 1, "box"), (48, 64, 5, "pbc")]
 
 
-@pytest.mark.parametrize("small", [0, 300, 2000])
+@pytest.mark.parametrize("small", [0, 300, 2000, 5000])
 @pytest.mark.parametrize("grid", GRIDS)
 def test_paths_match_oracle(gpu_lib, grid, small):
     from jd_lepic_b200.simulation import GpuSimulation
