@@ -64,6 +64,7 @@ static void free_all(lepic_ctx *c) {
     if (c->ev_up) cudaEventDestroy(c->ev_up);
     F(c->snap);
     io_free(c);
+    free(c->mg_plan);
     if (c->stream) cudaStreamDestroy(c->stream);
 }
 
@@ -336,11 +337,15 @@ extern "C" int lepic_gpu_set_options(lepic_ctx *c, const lepic_options *in) {
     }
     // the work list of a cooperative launch depends on these: wait for launches in flight
     LCUDA(cudaStreamSynchronize(c->stream));
-    const bool relaunch = o.ctas_per_sm != c->opt.ctas_per_sm;
+    const bool relaunch = o.ctas_per_sm != c->opt.ctas_per_sm, replan = o.mg_small_nodes != c->opt.mg_small_nodes;
     c->opt = o;
     if (relaunch) {
         c->mg_grid_mixed = 0;  // sized again at the next mixed solve
         c->mg_grid_mixed64 = 0;
+    }
+    if (replan) {
+        const int r = mg_init(c);
+        if (r != LEPIC_OK) return r;
     }
     return LEPIC_OK;
 }

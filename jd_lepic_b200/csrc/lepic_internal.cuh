@@ -193,6 +193,7 @@ struct lepic_ctx {
     int nlev = 0;
     double *partials = nullptr;
     int mg_grid = 0, mg_grid_mixed = 0, mg_grid_mixed64 = 0;
+    void *mg_plan = nullptr;   // the FP64 multigrid's kernel parameters (mg.cu)
     double *cg_r = nullptr, *cg_p = nullptr, *cg_ap = nullptr;  // finest-level CG vectors
     // exact solve of the mixed cycle's on-chip top level: the inverse of that level's operator
     // (FP32, cn x cn, symmetric) and, per unknown, its node and right-hand-side indices

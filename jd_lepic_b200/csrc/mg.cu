@@ -862,12 +862,14 @@ __global__ void __launch_bounds__(MGT, 1) k_mg_solve(const __grid_constant__ MGP
 // are 5 % of the 384 x 256 solve faster on CTA 0, 33^2 nodes 10 % of the 128^2 solve.
 #define MG_SMEM (224 * 1024)   // dynamic shared memory per CTA (one per SM)
 
-static MGP mg_params(lepic_ctx *c, double eps, int mode) {
+// The kernel's parameters but for a solve's own (mg_solve): the split of the levels and their tiles,
+// which follow from the deck and the options and take about 6 us per tiled level to choose.
+static MGP mg_params(const lepic_ctx *c) {
     MGP P;
     memset(&P, 0, sizeof(P));
     const double eps0 = c->cfg.eps0;
     for (int l = 0; l < c->nlev; l++) {
-        MGLevel &a = c->lev[l];
+        const MGLevel &a = c->lev[l];
         MGDev &d = P.L[l];
         d.nx = a.nx; d.ny = a.ny;
         d.aw = eps0 / (a.hx * a.hx);
@@ -917,34 +919,39 @@ static MGP mg_params(lepic_ctx *c, double eps, int mode) {
             }
     }
     P.omega = c->cfg.omega;
-    P.eps = eps;
     P.alpha = fabs((double)(c->cfg.nx + 1) * (c->cfg.ny + 1) * P.L[0].ac) * 1.0;
     P.ncycl = c->cfg.ncycl;
     P.pbc = c->cfg.flag_pbc;
     P.nmn = c->cfg.flag_nmn;
-    P.mode = mode;
     P.partials = c->partials;
     P.cnt = c->dcnt;
-    P.bar_extra = (unsigned)c->opt.barrier_extra;
     return P;
 }
 
+// the plan of a context's solves: at its creation, and again when an option it depends on changes
 int mg_init(lepic_ctx *c) {
     int occ = 0;
     LCUDA(cudaFuncSetAttribute(k_mg_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM));
     LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mg_solve, MGT, MG_SMEM));
     if (occ < 1) { c->last_err = "multigrid kernel does not fit on an SM"; return LEPIC_ECUDA; }
     c->mg_grid = c->num_sms;       // a CTA takes an SM's shared memory
-    return LEPIC_OK;
-}
-
-int mg_solve(lepic_ctx *c, double eps, int mode) {
-    MGP P = mg_params(c, eps, mode);
+    const MGP P = mg_params(c);
     for (int l = P.Ls; l < P.ng; l++)
         if (c->lev[l].u2_len < mg_level_len(P.L[l].nx, P.L[l].ny)) {   // a stage keeps its start there
             c->last_err = "multigrid: a level's second buffer is too short";
             return LEPIC_ECUDA;
         }
+    if (!c->mg_plan && !(c->mg_plan = malloc(sizeof(MGP)))) { c->last_err = "multigrid: no memory for its plan"; return LEPIC_ENOMEM; }
+    memcpy(c->mg_plan, &P, sizeof(P));
+    return LEPIC_OK;
+}
+
+int mg_solve(lepic_ctx *c, double eps, int mode) {
+    MGP P;
+    memcpy(&P, c->mg_plan, sizeof(P));
+    P.eps = eps;
+    P.mode = mode;
+    P.bar_extra = (unsigned)c->opt.barrier_extra;
     void *args[] = {&P};
     LCUDA(cudaMemsetAsync(&c->dcnt->bar_arrived, 0, sizeof(unsigned long long) + sizeof(int), c->stream));
     LCUDA(cudaLaunchCooperativeKernel((void *)k_mg_solve, dim3(P.Ls == 0 ? 1 : c->mg_grid), dim3(MGT), args, MG_SMEM, c->stream));
