@@ -152,10 +152,17 @@ __global__ void k_scan_final(const int *counts, long long n, const int *blocksum
 // particle that changed cell inside its old tile is met by the same warp in slot order as the
 // particles of its new cell, so its position comes out in stable order; only a cell that
 // receives particles from another work unit (a neighbouring tile, the tail) can come out of
-// order, and the segment sort below checks every segment and sorts those.  (Fixed 1024-slot
-// chunks cut every tile into pieces, so a particle moving to the next row of cells reached
-// another chunk and nearly every electron cell needed the segment sort.)  Units are dispensed
-// dynamically: the items' sizes follow the density.
+// order, and the segment sort below checks every segment and sorts those.  So a unit's size weighs
+// warps at work against segments out of order: a cut through a tile sends a particle that moves to
+// the next row of cells to another unit.  The units are the push's (push_chunk()): 512 slots and up
+// on small grids, where 16384 leave most of the GPU idle, whole tiles or large pieces on large ones.
+// Whole sorts of electrons / ions after ten steps, against units of up to 16384: 128^2 cells at 100 per
+// cell 313 / 124 us against 327 / 171, 384 x 256 periodic at 60 291 / 166 against 314 / 228, 600 x 363 at
+// 50 248 / 155 against 275 / 198; on 1024 x 512 at 100, whose tiles fall into three pieces instead of
+// two, 1275 / 475 against 1110 / 495, less than the ten pushes between gain (9.45 against 9.74 ms).
+// (Fixed chunks of 1024 slots, cut without regard to tiles at every size, needed the segment sort for
+// nearly every electron cell at 2048^2.)  Units are dispensed dynamically: the items' sizes follow
+// the density.
 #define SCATTER_CHUNK 1024
 #define SCATTER_STEPS 8
 __global__ void k_scatter(const int *keys, const WorkItem *items, DevCounters *cnt, int sp, int *cursor, int *perm) {
