@@ -97,16 +97,25 @@ def test_free_right_column_between_periodic_edges(gpu_lib, size, small):
         s.close()
 
 
-def test_quotient_of_extreme_values(gpu_lib):
-    """The update divides by the fixed diagonal with a corrected reciprocal where the dividend is in
-    range and with the general division elsewhere: sources from 1e-300 to 1e200 in one deck."""
+# cell sizes (m) with unrelated mantissas of the diagonal, one whose diagonal lies above 1e30 on all
+# levels but the coarsest, one below 1e-30 on all of them: there the general division takes every dividend
+CELLS = [(1e-4, 1e-4, (1e-300, 1e-150, 1.0, 1e150, 1e280)), (1.371e-4, 0.733e-4, (1e-300, 1.0, 1e280)),
+         (3.1e-5, 2.9e-5, (1e-150, 1.0, 1e272)), (1e-21, 1.3e-21, (1e-150, 1.0, 1e150)), (1e10, 1.7e10, (1e-150, 1.0, 1e150))]
+
+
+@pytest.mark.parametrize("cell", CELLS)
+def test_quotient_of_extreme_values(gpu_lib, cell):
+    """The update divides by the fixed diagonal with a corrected reciprocal where dividend and
+    diagonal are in range (2^-899 to 2^901, 1e-30 to 1e30) and with the general division elsewhere:
+    sources from 1e-300 to 1e280 beside nodes that are zero, bit for bit."""
     from jd_lepic_b200.simulation import GpuSimulation
     nx = ny = 32
     case = _case(nx, ny, 4, "box")
+    case.dx, case.dy = cell[0], cell[1]
     case.phi0 = np.zeros_like(case.phi0)
     s = GpuSimulation(case, tile=(8, 8), load=False, capacity=64, config={"ncycl": 1})
     try:
-        for scale in (1e-300, 1e-150, 1.0, 1e150):
+        for scale in cell[2]:
             rhs = np.zeros((ny + 1, nx + 1))
             rhs[5, 7], rhs[20, 11] = scale, -3.0 * scale
             a = np.ascontiguousarray(rhs)
@@ -118,6 +127,7 @@ def test_quotient_of_extreme_values(gpu_lib):
             got = s.grid(capi.GRID_PHI)
             ref = case.phi0.copy()
             O.solve(O.make_cfg(case, s.sp), ref, rhs, case.bcnd, 4, 1e-320, ncycl=1)
+            assert np.isfinite(ref).all() and np.abs(ref).max() > 0.0
             assert np.array_equal(got, ref)
     finally:
         s.close()
