@@ -143,3 +143,34 @@ def test_learned_warm_start_saves_iterations(gpu_lib):
     assert max(ratios) < 0.5, ratios
     assert sum(learned) <= sum(plain) and min(learned) < max(plain), (plain, learned)
     s.close()
+
+
+def test_learned_start_changes_no_solution(gpu_lib):
+    """The solution after a learned start is solved to the tolerance by the restatement's own residual,
+    and is the plain solver's: A e = r1 - r2 with residuals below eps ||b||, so ||e|| <= 2 eps ||b|| / l
+    with l the smallest eigenvalue of the grounded box (the plate only raises it)."""
+    from jd_lepic_b200.simulation import GpuSimulation
+    case = configs.case4(ppc=20, nx=128, ny=128)
+    s = GpuSimulation(case, tile=(16, 16))
+    cfg = capi.LepicCnnConfig(enable_training=1, warmup_solves=4, steps_warmup=2, train_every=1, steps_after=1,
+                              crop=64, batch=4, lr=C.c_float(2e-3), seed=5)
+    try:
+        s.check(s.lib.lepic_gpu_cnn_configure(s.ctx, C.byref(cfg)), "cnn_configure")
+        for it in range(2, 10):
+            s.check(s.lib.lepic_gpu_step(s.ctx, it, 1e-8, capi.POISSON_LEARNED), "step")
+        rhs = s.calc_rhs()
+        prev = s.grid(capi.GRID_PHI).copy()
+        plain = s.solve(eps=1e-8, mode=capi.POISSON_MIXED_IR, phi=prev)["phi"]
+        st = s.solve(eps=1e-8, mode=capi.POISSON_LEARNED, phi=prev)
+        ocfg = O.make_cfg(case, s.sp)
+        assert O.l2_residual(ocfg, prev, rhs, case.bcnd) > 1e-8      # there is something to solve
+        for phi in (plain, st["phi"]):
+            assert O.l2_residual(ocfg, phi, rhs, case.bcnd) <= 1e-8 * (1 + 1e-4)
+        w = np.where(case.bcnd > 0, prev, 0.0)
+        lap = lambda v: ((v[1:-1, :-2] + v[1:-1, 2:]) / case.dx ** 2 + (v[2:, 1:-1] + v[:-2, 1:-1]) / case.dy ** 2)  # noqa: E731
+        norm = np.linalg.norm((rhs - ocfg.eps0 * lap(w))[case.bcnd[1:-1, 1:-1] == -1])
+        low = ocfg.eps0 * sum(4 / h ** 2 * np.sin(np.pi / (2 * n)) ** 2 for h, n in ((case.dx, case.nx), (case.dy, case.ny)))
+        diff = np.linalg.norm(st["phi"] - plain)
+        assert diff <= 2e-8 * norm / low * (1 + 1e-3), (diff, 2e-8 * norm / low, np.linalg.norm(plain))
+    finally:
+        s.close()
