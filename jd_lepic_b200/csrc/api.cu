@@ -215,6 +215,7 @@ static int create_impl(lepic_ctx *c, const lepic_config *cfg, const int32_t *bcn
             LCUDA(cudaMemcpy(L.bc, cur.data(), nnl, cudaMemcpyHostToDevice));
             prev.swap(cur);
         }
+        for (int i = 1; i <= L.nx + 1; i++) L.top_counts = L.top_counts || prev[i + (size_t)(L.ny + 1) * (L.nx + 3)] == -1;
         LALLOC(L.e32, nnl); LALLOC(L.e32b, nnl); LALLOC(L.r32, (size_t)(L.nx + 1) * (L.ny + 1));
         LCUDA(cudaMemset(L.e32, 0, sizeof(float) * nnl));
         LCUDA(cudaMemset(L.e32b, 0, sizeof(float) * nnl));

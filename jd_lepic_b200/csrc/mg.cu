@@ -41,6 +41,7 @@ struct MGDev {
     double *b;
     const int8_t *bc;
     int tx, ty;           // the tile of the level's passes
+    int seam;             // its residuals are final only after the edge rows' copy: summed in a pass of their own
     int su, sb, sm;       // levels of the CTA-0 part: offsets of u, b (doubles) and the mask (bytes)
 };
 
@@ -138,11 +139,6 @@ __device__ __forceinline__ Patch tile_patch(const MGP &P, const MGDev &L, int ti
     g.mo = 8 * (MG_SLOTS + 2 * P.cap);
     return g;
 }
-
-// With an odd number of rows between periodic edges the nodes across the edge have the colour of
-// their neighbours, so a half-sweep's residuals are not final before the edge rows are copied:
-// such a level (only the coarsest of a deck can be one) sums them in a pass of their own.
-__device__ __forceinline__ bool odd_seam(int pbc, int ny) { return pbc && (ny & 1); }
 
 // a whole level in CTA 0's shared memory
 __device__ __forceinline__ Patch level_patch(const MGP &P, int l) {
@@ -442,7 +438,7 @@ __device__ __forceinline__ void team_sync(int T) {
 // (columns there are updated like the rest; what they hold reaches no further either).
 __device__ __forceinline__ void sweeps(const MGP &P, const Patch &g, const MGDev &L, int K, int T, bool l2, bool add) {
     double *const slot = smd + threadIdx.x;
-    const bool pbc = P.pbc != 0, seam = odd_seam(P.pbc, L.ny);
+    const bool pbc = P.pbc != 0, seam = L.seam != 0;
     const Coef k{L.aw, L.an, L.ac, L.y, P.omega, 1.0 - P.omega};
     const Plane red = plane_of(g, 0), black = plane_of(g, 1);
     const int RP = g.RP, RH = g.RH, c0 = g.clip0, c1 = g.clip1;
@@ -877,6 +873,11 @@ static MGP mg_params(const lepic_ctx *c) {
         d.ac = -(d.an + d.an + d.aw + d.aw);
         d.y = fabs(d.ac) > 1e-30 && fabs(d.ac) < 1e30 ? 1.0 / d.ac : 0.0;
         d.u = a.u; d.b = a.b; d.bc = a.bc;
+        // With an odd number of rows between periodic edges (only the coarsest level of a deck can
+        // have one) the nodes across the edge have the colour of their neighbours, and nodes of row
+        // ny + 1 whose residual counts are overwritten by the copy after their update: in both cases
+        // a half-sweep's residuals are not final before the edge rows are copied
+        d.seam = c->cfg.flag_pbc && ((a.ny & 1) || a.top_counts);
         d.u2 = l == 0 ? c->cg_ap : a.u2;
     }
     P.ng = c->nlev;

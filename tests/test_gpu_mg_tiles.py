@@ -97,6 +97,38 @@ def test_free_right_column_between_periodic_edges(gpu_lib, size, small):
         s.close()
 
 
+@pytest.mark.parametrize("small", [0, 300, 2000])
+@pytest.mark.parametrize("size", [(32, 24, 3), (64, 48, 4), (96, 72, 4)])
+def test_counted_nodes_on_the_copied_edge_row(gpu_lib, size, small):
+    """Label -1 on the upper edge row of a periodic deck: its nodes' residuals count, and the copy of
+    row 1 overwrites them after each half-sweep.  They never vanish, so the cycles run out; residual
+    and potential are the restatement's."""
+    from jd_lepic_b200.simulation import GpuSimulation
+    nx, ny, ng = size
+    case = _case(nx, ny, ng, "pbc")
+    case.bcnd[ny + 1, 2:nx + 1] = -1
+    case.phi0 = configs.potentials(case.bcnd, {1: 5.0, 2: 10.0})
+    s = GpuSimulation(case, tile=(8, 8), load=False, capacity=64, config={"ncycl": 6})
+    try:
+        s.set_options(mg_small_nodes=small)
+        rng = np.random.default_rng(nx)
+        X, Y = np.meshgrid(np.arange(nx + 1) / nx, np.arange(ny + 1) / ny)
+        rhs = 1.6e-3 * np.sin(3 * np.pi * X) * np.cos(2 * np.pi * Y) + 2e-4 * rng.normal(size=X.shape)
+        a = np.ascontiguousarray(rhs)
+        s.check(s.lib.lepic_gpu_set_grid(s.ctx, capi.GRID_RHS, a.ctypes.data_as(C.POINTER(C.c_double))), "set_grid")
+        s.set_phi(case.phi0)
+        st = capi.LepicSolveStats()
+        rc = s.lib.lepic_gpu_iterative_solver(s.ctx, None, 0.02, capi.POISSON_FP64_MG, C.byref(st))
+        ref = case.phi0.copy()
+        orc, ost = O.solve(O.make_cfg(case, s.sp), ref, rhs, case.bcnd, ng, 0.02, ncycl=6)
+        assert rc == capi.ENOTCONV and orc == 0 and ost.k == 6
+        assert (st.cycles, st.sweeps_fine) == (ost.k, ost.sweeps_fine)
+        assert abs(st.res_l1 - ost.res) <= 1e-12 * ost.res
+        assert np.abs(s.grid(capi.GRID_PHI) - ref).max() <= 1e-13 * np.abs(ref).max()
+    finally:
+        s.close()
+
+
 # cell sizes (m) with unrelated mantissas of the diagonal, one whose diagonal lies above 1e30 on all
 # levels but the coarsest, one below 1e-30 on all of them: there the general division takes every dividend
 CELLS = [(1e-4, 1e-4, (1e-300, 1e-150, 1.0, 1e150, 1e280)), (1.371e-4, 0.733e-4, (1e-300, 1.0, 1e280)),
