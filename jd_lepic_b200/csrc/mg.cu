@@ -336,10 +336,8 @@ __device__ __forceinline__ void restriction(const Patch &g, int pbc, int ro, Mas
     const int lg = lanes_of(ic1 - ic0), lpr = 1 << lg;
     const int lane = threadIdx.x & (lpr - 1), sub = threadIdx.x >> lg, nsub = MGT >> lg;
     const int lny = g.wrap == 3 ? ny : ny - g.a0;    // local row of ny (periodic)
-    // r_pbc(x) of mg.f90:298-311 (zero where the reference leaves it unset, and one past its end,
-    // which a free node of the right column asks for)
+    // r_pbc(x) of mg.f90:298-311 (zero where the reference leaves it unset)
     auto rpbc = [&](int x) {
-        if (x > nx + 1) return 0.0;
         const int t = (lny + 1) * RP + x - g.ri0;
         bool set;
         if (x & 1) set = g.m(t) <= 0;
@@ -362,7 +360,7 @@ __device__ __forceinline__ void restriction(const Patch &g, int pbc, int ro, Mas
                     if (m(1) <= 0) r2 = r(1);
                 if (m(1 - RP) <= 0) {
                     if (ir != nx + 1 && jr != 1) r3 = r(1 - RP);
-                    else if (jr == 1) r3 = pbc ? rpbc(ir + 1) : 0.0;
+                    else if (jr == 1) r3 = pbc && ir <= nx ? rpbc(ir + 1) : 0.0;   // zero past a free right column too
                 }
                 if (m(-RP) <= 0) {
                     if (jr != 1) r4 = r(-RP);
